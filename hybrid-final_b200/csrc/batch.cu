@@ -92,18 +92,24 @@ hp_status batch_dev_build(hp_case *const *cases, int n, BatchDev &b) {
     for (int m = 0; m < 5; m++)
         for (int k = 0; k <= m; k++) {
             b.list_off[m][k] = (int)lists.size();
+            b.list_per[m][k] = b.list_ngy[m][k] = 0;
             for (int i = 0; i < n; i++) {
                 if (cases[i]->h.field_mode == 2) continue; // separable inner solve, not PCG
                 if (cases[i]->pcg_cluster > 16) continue;  // whole-GPU solve, launched on its own
                 int cs = std::min(pcg_cluster_for_nodes(cases[i]->s.Gsize), 1 << m);
-                if (cs == (1 << k)) lists.push_back(i);
+                if (cs != (1 << k)) continue;
+                lists.push_back(i);
+                b.list_per[m][k] = std::max(b.list_per[m][k], (cases[i]->s.Gsize + cs - 1) / cs);
+                b.list_ngy[m][k] = std::max(b.list_ngy[m][k], cases[i]->s.ngy);
             }
             b.list_n[m][k] = (int)lists.size() - b.list_off[m][k];
         }
     b.grid_cases.clear();
     for (int i = 0; i < n; i++)
         if (cases[i]->h.field_mode != 2 && cases[i]->pcg_cluster > 16) {
-            b.grid_cases.push_back({(int)lists.size(), cases[i]->pcg_cluster});
+            const int cs = cases[i]->pcg_cluster;
+            b.grid_cases.push_back(PcgGroup{cs, 0, nullptr, (int)lists.size(), (cases[i]->s.Gsize + cs - 1) / cs,
+                                            cases[i]->s.ngy});
             lists.push_back(i);
         }
     {
@@ -128,8 +134,10 @@ std::vector<PcgGroup> BatchDev::groups(int cluster_max, int block) const {
     while ((1 << (m + 1)) <= cluster_max && m < 4) m++;
     std::vector<PcgGroup> g;
     for (int k = 0; k <= m; k++)
-        if (list_n[m][k] > 0) g.push_back(PcgGroup{1 << k, block, d_lists + list_off[m][k], list_n[m][k]});
-    for (const auto &gc : grid_cases) g.push_back(PcgGroup{gc.second, block, d_lists + gc.first, 1});
+        if (list_n[m][k] > 0)
+            g.push_back(PcgGroup{1 << k, block, d_lists + list_off[m][k], list_n[m][k], list_per[m][k], list_ngy[m][k]});
+    for (const PcgGroup &gc : grid_cases)
+        g.push_back(PcgGroup{gc.cluster, block, d_lists + gc.n, 1, gc.max_per, gc.max_ngy});
     return g;
 }
 

@@ -518,7 +518,13 @@ hp_status build_device(hp_case *c) {
     // a PCG case too large for a 16-CTA cluster solves over the whole GPU
     // (cooperative launch); its CTA totals need 2 x 2 doubles per CTA
     const int grid_ctas = h.field_mode != 2 ? pcg_grid_ctas(G, c->lc.pcg_block) : 0;
-    if (grid_ctas > 0) TRY(dalloc(c, &h.pcg_part, 4 * (size_t)((G + 1023) / 1024)));
+    if (grid_ctas > 0) {
+        TRY(dalloc(c, &h.pcg_part, 4 * (size_t)((G + 1023) / 1024)));
+        const size_t most = std::min((G + 1023) / 1024, 512); // CTAs of any launch shape
+        TRY(dalloc(c, &h.pcg_slot, 4 * most * most));
+        TRY(dalloc(c, &h.pcg_edge, (size_t)G));
+        TRY(dalloc(c, &h.pcg_seq, 1));
+    }
     TRY(dalloc(c, &c->d_list0, 1));
     TRY(dalloc(c, &c->d_case, 1));
     CK(cudaMemcpy(c->d_case, &h, sizeof(h), cudaMemcpyHostToDevice));
@@ -553,7 +559,8 @@ cudaStream_t as_stream(void *s) { return (cudaStream_t)s; }
 
 
 hp_status op_field(hp_case *c, cudaStream_t st) {
-    PcgGroup g{c->pcg_cluster, c->lc.pcg_block, c->d_list0, 1};
+    PcgGroup g{c->pcg_cluster, c->lc.pcg_block, c->d_list0, 1, (c->s.Gsize + c->pcg_cluster - 1) / c->pcg_cluster,
+               c->s.ngy};
     const bool fast = c->h.field_mode == 2;
     cudaError_t e = launch_field(c->d_case, c->d_items + 4, 1, c->s.Gsize, &g, fast ? 0 : 1,
                                  fast ? &c->fplan.plan : nullptr, st, c->h.cs != nullptr);

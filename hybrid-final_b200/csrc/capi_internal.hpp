@@ -87,7 +87,8 @@ struct BatchDev {
     // cluster size, concatenated in d_lists
     int *d_lists = nullptr;
     int list_off[5][5] = {}, list_n[5][5] = {};
-    std::vector<std::pair<int, int>> grid_cases; // whole-GPU PCG cases: (offset in the lists, CTAs)
+    int list_per[5][5] = {}, list_ngy[5][5] = {}; // most nodes per CTA and grid rows of a list's cases
+    std::vector<hp::PcgGroup> grid_cases; // whole-GPU PCG cases, one group each; n: the case's offset in the lists
     std::vector<hp::PcgGroup> groups(int cluster_max, int block) const;
     FastPlanDev fast;
 };

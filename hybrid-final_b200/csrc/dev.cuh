@@ -100,6 +100,11 @@ struct DevCase {
     double *x64, *b64;              // [G] FP64 solution and right-hand side
     double *dots;                   // scratch for cluster reductions [64]
     double *pcg_part;               // [2 x 2 x CTAs] CTA totals of the cooperative grid solve (null: cluster)
+    // exchanges of the on-chip whole-GPU solve (null: cluster): words of 32 bits of data under 32 bits of
+    // exchange number
+    unsigned long long *pcg_slot;   // [2 x CTAs x CTAs x 2] inboxes of the CTA totals (two words each), two exchanges in turn
+    unsigned long long *pcg_edge;   // [G] residuals of the nodes at the edges of the CTAs' ranges
+    unsigned *pcg_seq;              // the last exchange's number
     double *den;                    // [nsp*G]
     double *source;                 // [G]
     double4 *cw[DMAXSP];            // [C] per-cell corner weight sums

@@ -13,7 +13,7 @@ namespace hp {
 namespace dv {
 
 constexpr unsigned FULL = 0xffffffffu;
-constexpr uint32_t ST_OVERFLOW = 0x1u, ST_NONFINITE = 0x2u, ST_NOCONV = 0x4u, ST_WALK = 0x10u, ST_SURFACE = 0x20u;
+constexpr uint32_t ST_OVERFLOW = 0x1u, ST_NONFINITE = 0x2u, ST_NOCONV = 0x4u, ST_TIMEOUT = 0x8u, ST_WALK = 0x10u, ST_SURFACE = 0x20u;
 
 __device__ __forceinline__ int find_case(const int *start, int n, int w) {
     int lo = 0, hi = n;
@@ -49,6 +49,39 @@ __device__ __forceinline__ int lower_lane_hits(unsigned mask4, unsigned lt, int 
         total += __popc(b);
     }
     return pre;
+}
+
+// sum over the warp by the xor tree, the same bits on every lane
+__device__ __forceinline__ double warp_sum_d(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
+    return v;
+}
+
+// ------------------------------------------------------------------ the 5-point operator at node n
+__device__ __forceinline__ float spmv_f(const float *__restrict__ st, int G, int ngy, int n,
+                                        const float *__restrict__ v) {
+    // CSR order of the reference rows: W, S, C, N, E (src/load.c:170-240)
+    float out = 0.0f;
+    const float cw = st[n], cs = st[G + n], cc = st[2 * G + n], cn = st[3 * G + n], ce = st[4 * G + n];
+    if (cw != 0.0f) out += cw * v[n - ngy];
+    if (cs != 0.0f) out += cs * v[n - 1];
+    out += cc * v[n];
+    if (cn != 0.0f) out += cn * v[n + 1];
+    if (ce != 0.0f) out += ce * v[n + ngy];
+    return out;
+}
+
+__device__ __forceinline__ double spmv_d(const float *__restrict__ st, int G, int ngy, int n,
+                                         const double *__restrict__ v) {
+    double out = 0.0;
+    const float cw = st[n], cs = st[G + n], cc = st[2 * G + n], cn = st[3 * G + n], ce = st[4 * G + n];
+    if (cw != 0.0f) out += (double)cw * v[n - ngy];
+    if (cs != 0.0f) out += (double)cs * v[n - 1];
+    out += (double)cc * v[n];
+    if (cn != 0.0f) out += (double)cn * v[n + 1];
+    if (ce != 0.0f) out += (double)ce * v[n + ngy];
+    return out;
 }
 
 // ------------------------------------------------------------------ MCC helpers

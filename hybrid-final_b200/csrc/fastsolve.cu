@@ -11,6 +11,7 @@
 // --fmad=false), so a CPU loop reproduces it exactly.
 #include <cstdint>
 
+#include "devutil.cuh"
 #include "kernels.cuh"
 #include "prof.cuh"
 

@@ -1173,12 +1173,6 @@ __global__ void __launch_bounds__(MCC_TPB, MCC_MINB) k_mcc_ar(const DevCase *__r
 // DepositAtom (src/cuda_Deposit.cu:289-317): per-cell sums of the four CIC
 // weights; lanes accumulate in FP32, the warp reduces in FP64 and writes one
 // double4 per cell, which the node pass gathers in a fixed order.
-__device__ __forceinline__ double warp_sum_d(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-    return v;
-}
-
 // DEP_G consecutive (species, cell) items per warp: lanes 0..G-1 resolve
 // their item's case, count and array bases together, every lane then loads
 // its first slot of all G cells at once, and the cells are summed one after
@@ -1380,32 +1374,6 @@ __global__ void __launch_bounds__(256) k_source(const DevCase *__restrict__ case
 }
 
 // ------------------------------------------------------------------ Field
-__device__ __forceinline__ float spmv_f(const float *__restrict__ st, int G, int ngy, int n, int i, int j, int ngx,
-                                        const float *__restrict__ v) {
-    // CSR order of the reference rows: W, S, C, N, E (src/load.c:170-240)
-    float out = 0.0f;
-    const float cw = st[n], cs = st[G + n], cc = st[2 * G + n], cn = st[3 * G + n], ce = st[4 * G + n];
-    if (cw != 0.0f) out += cw * v[n - ngy];
-    if (cs != 0.0f) out += cs * v[n - 1];
-    out += cc * v[n];
-    if (cn != 0.0f) out += cn * v[n + 1];
-    if (ce != 0.0f) out += ce * v[n + ngy];
-    (void)i; (void)j; (void)ngx;
-    return out;
-}
-
-__device__ __forceinline__ double spmv_d(const float *__restrict__ st, int G, int ngy, int n,
-                                         const double *__restrict__ v) {
-    double out = 0.0;
-    const float cw = st[n], cs = st[G + n], cc = st[2 * G + n], cn = st[3 * G + n], ce = st[4 * G + n];
-    if (cw != 0.0f) out += (double)cw * v[n - ngy];
-    if (cs != 0.0f) out += (double)cs * v[n - 1];
-    out += (double)cc * v[n];
-    if (cn != 0.0f) out += (double)cn * v[n + 1];
-    if (ce != 0.0f) out += (double)ce * v[n + ngy];
-    return out;
-}
-
 // CTAs of the whole-GPU solve, at most
 constexpr int PCG_GRID_MAX = 512;
 
@@ -1526,7 +1494,7 @@ __global__ void __launch_bounds__(512) k_pcg(const DevCase *__restrict__ cases, 
     const int li = GRID ? 0 : (int)blockIdx.x / CS;
     if (li >= nlist) return;
     const DevCase &d = cases[list[li]];
-    const int G = d.G, ngy = d.ngy, ngx = d.ngx;
+    const int G = d.G, ngy = d.ngy;
     const int per = (G + CS - 1) / CS;
     const int lo = rank * per, hi = min(G, lo + per);
     const int T = blockDim.x;
@@ -1614,7 +1582,7 @@ __global__ void __launch_bounds__(512) k_pcg(const DevCase *__restrict__ cases, 
         for (int n = lo + threadIdx.x; n < hi; n += T) {
             const float cc = st[2 * G + n];
             if (cc == 0.0f) continue;
-            const float ax = spmv_f(st, G, ngy, n, 0, 0, ngx, x);
+            const float ax = spmv_f(st, G, ngy, n, x);
             const float rr = -1.0f * ax + (float)d.b64[n];
             r[n] = rr;
             const float z = (1 / cc) * rr;
@@ -2161,8 +2129,7 @@ cudaError_t launch_move(const DevCase *cases, const int *item_start, int ncases,
     if (lc.move_unroll == 2) k_move_u<2><<<nb, tpb, 0, st>>>(cases, item_start, ncases, items);
     else if (lc.move_unroll == 4) k_move_u<4><<<nb, tpb, 0, st>>>(cases, item_start, ncases, items);
     else
-        k_move<MOVE_RING><<<nb, tpb, (size_t)(tpb / 32) * MOVE_RING * 5 * 32 * sizeof(float), st>>>(
-            cases, item_start, ncases, items);
+        k_move<MOVE_RING><<<nb, tpb, (size_t)(tpb / 32) * MOVE_RING * 5 * 32 * sizeof(float), st>>>(cases, item_start, ncases, items);
     return cudaGetLastError();
 }
 
@@ -2186,13 +2153,11 @@ cudaError_t launch_sort(const DevCase *cases, const int *item_start, int ncases,
     // and Deposit prefer smaller blocks
     const int tpb = 32 * std::min(std::max(lc.warps_per_block, 8), SORT_MAXW);
     prof::mark(st, "k_sort_push");
-    k_sort_push<<<blocks_for((long long)items * 32, tpb), tpb, (size_t)(tpb / 32) * SORT_PRE * SORT_SLOT * sizeof(float),
-                  st>>>(cases, item_start, ncases, items);
+    k_sort_push<<<blocks_for((long long)items * 32, tpb), tpb, (size_t)(tpb / 32) * SORT_PRE * SORT_SLOT * sizeof(float), st>>>(cases, item_start, ncases, items);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     prof::mark(st, "k_sort_count");
-    k_sort_count<<<blocks_for((long long)(items + 31) / 32 * 32, tpb), tpb, 0, st>>>(cases, item_start, ncases,
-                                                                                     items);
+    k_sort_count<<<blocks_for((long long)(items + 31) / 32 * 32, tpb), tpb, 0, st>>>(cases, item_start, ncases, items);
     return cudaGetLastError();
 }
 
@@ -2215,8 +2180,7 @@ cudaError_t launch_deposit(const DevCase *cases, const int *cell_items, const in
     const int tpb = 32 * std::min(std::max(lc.warps_per_block, 1), 16);
     if (n_cell_items > 0) {
         prof::mark(st, "k_deposit_cells");
-        k_deposit_cells<<<blocks_for((long long)(n_cell_items + DEP_G - 1) / DEP_G * 32, tpb), tpb, 0, st>>>(cases, cell_items, ncases,
-                                                                                        n_cell_items);
+        k_deposit_cells<<<blocks_for((long long)(n_cell_items + DEP_G - 1) / DEP_G * 32, tpb), tpb, 0, st>>>(cases, cell_items, ncases, n_cell_items);
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
@@ -2268,6 +2232,10 @@ cudaError_t launch_field(const DevCase *cases, const int *node_items, int ncases
     for (int g = 0; g < ngroups; g++) {
         const PcgGroup &pg = groups[g];
         if (pg.n <= 0) continue;
+        bool done = false;
+        cudaError_t ec = launch_pcg_chip(cases, pg, st, done);
+        if (ec != cudaSuccess) return ec;
+        if (done) continue;
         if (pg.cluster > 16) { // one cooperative launch per case over pg.cluster CTAs
             for (int k = 0; k < pg.n; k++) {
                 cudaLaunchConfig_t cfg = {};

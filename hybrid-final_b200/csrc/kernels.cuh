@@ -48,7 +48,11 @@ struct PcgGroup {
     int block;        // threads per CTA
     const int *list;  // device array of case indices
     int n;
+    int max_per, max_ngy; // most nodes per CTA and grid rows of its cases
 };
+// the solve with its state on chip (pcg.cu); done = false where the group's
+// launch shape is outside its range
+cudaError_t launch_pcg_chip(const DevCase *cases, const PcgGroup &pg, cudaStream_t st, bool &done);
 // field_mode 2 (fastsolve.cu): refinement passes with the separable inverse
 struct GemmProb {
     int M, N, K;
