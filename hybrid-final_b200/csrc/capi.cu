@@ -266,7 +266,19 @@ hp_status build_device(hp_case *c) {
     h.gas = s.main_gas; h.cond_numr = s.cond_numr; h.n_unknowns = s.n_unknowns;
     h.dt_dx = s.dt_dx; h.dt_dy = s.dt_dy; h.dt = s.dt;
     h.dx = s.dx; h.dy = s.dy; h.idx = s.idx; h.idy = s.idy; h.hdx = s.hdx; h.hdy = s.hdy; h.idxy = s.idxy;
+    h.div_c = FastDiv::of((unsigned)C);
+    h.div_ncy = FastDiv::of((unsigned)s.ncy);
     TRY(dupload(c, (int **)&h.sidx, s.sidx));
+    {
+        std::vector<uint8_t> open3(C, 0);
+        for (int i = 1; i + 1 < s.ncx; i++)
+            for (int j = 1; j + 1 < s.ncy; j++) {
+                bool open = true;
+                for (int q = 0; q < 9; q++) open = open && s.sidx[(size_t)(i + q / 3) * (s.ncy + 2) + (j + q % 3)] == 0;
+                open3[(size_t)i * s.ncy + j] = open;
+            }
+        TRY(dupload(c, (uint8_t **)&h.open3, open3));
+    }
     TRY(dupload(c, (int **)&h.boundary, s.boundary));
     TRY(dupload(c, (int **)&h.face, s.face));
     TRY(dupload(c, (int **)&h.cond_id, s.cond_id));
@@ -321,10 +333,8 @@ hp_status build_device(hp_case *c) {
         sp.Escale = s.sp[isp].Escale;
         sp.np2c = s.sp[isp].np2c;
         size_t nslot = (size_t)C * sp.cap;
-        TRY(dalloc(c, &sp.x, nslot));
-        TRY(dalloc(c, &sp.y, nslot));
-        TRY(dalloc(c, &sp.vx, nslot));
-        TRY(dalloc(c, &sp.vy, nslot));
+        TRY(dalloc(c, &sp.xy, nslot));
+        TRY(dalloc(c, &sp.v, nslot));
         TRY(dalloc(c, &sp.vz, nslot));
         TRY(dalloc(c, &sp.code, nslot));
         TRY(dalloc(c, &sp.cnt, C));
@@ -1098,16 +1108,23 @@ hp_status hp_get_particles(hp_case *c, int isp, int *counts, float *x, float *y,
     if (counts) std::memcpy(counts, cnt.data(), (size_t)C * 4);
     if (!x) return HP_OK;
     if (cap < total) return set_error("output arrays too small"), HP_ERR_ARG;
-    const size_t ns = (size_t)C * sp.cap;
-    std::vector<float> b(ns);
+    const float *srcs[3] = {(const float *)sp.xy, (const float *)sp.v, sp.vz};
     float *outs[5] = {x, y, vx, vy, vz};
-    float *srcs[5] = {sp.x, sp.y, sp.vx, sp.vy, sp.vz};
-    for (int a = 0; a < 5; a++) {
-        if (!outs[a]) continue;
-        CK(cudaMemcpy(b.data(), srcs[a], ns * 4, cudaMemcpyDeviceToHost));
+    std::vector<float> b;
+    for (int a = 0; a < 3; a++) { // the pairs (x, y) and (vx, vy), then vz
+        const size_t w = a < 2 ? 2 : 1;
+        float *o0 = outs[2 * a], *o1 = a < 2 ? outs[2 * a + 1] : nullptr;
+        if (!o0 && !o1) continue;
+        b.resize((size_t)C * sp.cap * w);
+        CK(cudaMemcpy(b.data(), srcs[a], b.size() * 4, cudaMemcpyDeviceToHost));
         size_t q = 0;
-        for (int cell = 0; cell < C; cell++)
-            for (int k = 0; k < cnt[cell]; k++) outs[a][q++] = b[(size_t)cell * sp.cap + k];
+        for (int cell = 0; cell < C; cell++) {
+            const float *from = b.data() + (size_t)cell * sp.cap * w;
+            for (int k = 0; k < cnt[cell]; k++, q++) {
+                if (o0) o0[q] = from[w * k];
+                if (o1) o1[q] = from[w * k + 1];
+            }
+        }
     }
     return HP_OK;
 }
@@ -1128,14 +1145,20 @@ hp_status hp_get_movers(hp_case *c, int isp, int *counts, float *x, float *y, fl
     if (!x) return HP_OK;
     if (cap < total) return set_error("output arrays too small"), HP_ERR_ARG;
     const size_t ns = (size_t)C * sp.cap;
-    std::vector<float> b(ns);
+    const float *srcs[3] = {(const float *)sp.xy, (const float *)sp.v, sp.vz};
     float *outs[5] = {x, y, vx, vy, vz};
-    float *srcs[5] = {sp.x, sp.y, sp.vx, sp.vy, sp.vz};
-    for (int a = 0; a < 5; a++) {
-        CK(cudaMemcpy(b.data(), srcs[a], ns * 4, cudaMemcpyDeviceToHost));
+    std::vector<float> b;
+    for (int a = 0; a < 3; a++) {
+        const size_t w = a < 2 ? 2 : 1;
+        b.resize(ns * w);
+        CK(cudaMemcpy(b.data(), srcs[a], b.size() * 4, cudaMemcpyDeviceToHost));
         size_t q = 0;
         for (int cell = 0; cell < C; cell++)
-            for (int r = 0; r < m[cell]; r++) outs[a][q++] = b[(size_t)cell * sp.cap + sp.cap - 1 - r];
+            for (int r = 0; r < m[cell]; r++, q++) {
+                const size_t at = ((size_t)cell * sp.cap + sp.cap - 1 - r) * w;
+                outs[2 * a][q] = b[at];
+                if (w == 2) outs[2 * a + 1][q] = b[at + 1];
+            }
     }
     if (codes) {
         std::vector<int8_t> cb(ns);

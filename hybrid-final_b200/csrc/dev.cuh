@@ -2,7 +2,11 @@
 //
 // HBM layout of one case (all arrays owned by the library):
 //   particles, per species s, structure of arrays over a cell-blocked slot pool:
-//     x[s][c*cap + k], y, vx, vy, vz    float   (x, y = offset inside cell c in [0,1))
+//     xy[s][c*cap + k]                  float2  (offset inside cell c in [0,1))
+//     v[s][c*cap + k]                   float2  (vx, vy)
+//     vz[s][c*cap + k]                  float
+//   (pairs: the push, the re-binning and the collisions read and write x with
+//   y and vx with vy, one address and one access each; the deposit reads xy alone)
 //     code[s][c*cap + k]                int8    (mover destination after Move)
 //     cnt[s][c]                         int32   particles resident in cell c
 //     nmov[s][c]                        int32   movers parked at the top of cell c
@@ -10,7 +14,7 @@
 //   cell c = i*ncy + j for the cell whose lower-left node is (i, j); the
 //   reference indexes the same cell by its node i*ngy + j and strides its
 //   slots by Gsize (src/cuda_Particle.cu:44-52).  Slots of one cell are
-//   contiguous here, so a warp that owns a cell reads 32 consecutive floats
+//   contiguous here, so a warp that owns a cell reads 32 consecutive entries
 //   per access.
 //   grid: Ex, Ey, phi (float, node layout), den (double, nsp*Gsize),
 //   source (double), PCG vectors in node layout (Gsize entries, non-unknown
@@ -32,8 +36,24 @@ constexpr int DMAXSP = 5;
 constexpr int DMAXCOND = 8;
 constexpr int DMAXSRC = 8;
 
+// n / d for n < 2^31 by a multiplication and a shift (Granlund & Montgomery,
+// Division by Invariant Integers using Multiplication, PLDI 1994, fig. 4.1)
+struct FastDiv {
+    unsigned mul, shift;
+    static FastDiv of(unsigned d) {
+        FastDiv f{0, 0};
+        while ((1ull << f.shift) < d) f.shift++;
+        f.mul = (unsigned)((((1ull << f.shift) - d) << 32) / d + 1);
+        return f;
+    }
+#ifdef __CUDACC__
+    __device__ __forceinline__ unsigned quot(unsigned n) const { return (__umulhi(mul, n) + n) >> shift; }
+#endif
+};
+
 struct DevSpecies {
-    float *x, *y, *vx, *vy, *vz;
+    float2 *xy, *v;
+    float *vz;
     int8_t *code;
     int *cnt;
     int *nmov;
@@ -69,7 +89,9 @@ struct DevCase {
     int ngx, ngy, ncx, ncy, G, C, nsp, gas, cond_numr, n_unknowns;
     float dt_dx, dt_dy, dt;
     float dx, dy, idx, idy, hdx, hdy, idxy;
+    FastDiv div_c, div_ncy; // by C and ncy
     const int *sidx;        // StructureIndex [(ncx+2)*(ncy+2)]
+    const uint8_t *open3;   // [C] 1: an inner cell whose 3x3 neighbourhood is all plasma (ghost code 0)
     const int *boundary, *face, *cond_id; // [G]
     const float *eps;       // [C] EPS0 * eps_r
     const float *dep_factor;// [G]

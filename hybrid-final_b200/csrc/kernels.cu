@@ -220,12 +220,7 @@ __device__ __forceinline__ int walk(const Geo d, int &i, int &j, float &lx, floa
     return 0;
 }
 
-// asynchronous global -> shared copies (LDGSTS): 4 bytes per lane, committed
-// per chunk; a lane waits for its own groups and reads only what it copied
-__device__ __forceinline__ void cp_async4(float *smem, const float *gmem) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
+// asynchronous global -> shared copies (LDGSTS) of 16 bytes, committed per chunk
 __device__ __forceinline__ void cp_async16(float *smem, const float *gmem) {
     const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
@@ -248,149 +243,171 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // 3x3 neighbourhood, CODE_FAR beyond it (also listed in the destination's
 // bucket as source<<18 | r), CODE_ABSORBED when it left
 // the domain.
-// The particle loads are asynchronous copies into a ring of R chunk slots per
-// warp in shared memory, so that R - 1 chunks of every warp are in flight
-// without holding registers.  vz is copied with the other arrays and written
-// back only where the slot changes: a per-particle load of it where needed
-// measured 4 % slower on the 257x129 case (148 vs 142 us) than the extra
-// 4 bytes per particle.
-constexpr int MOVE_RING = 4;
+//
+// It is bound by HBM as far as enough loads are in flight, and by instruction
+// issue beside that.  So a cell's chunks of 32 particles come through a ring
+// of R slots per warp in shared memory, filled by asynchronous copies R - 1
+// chunks ahead (no registers held: two chunks ahead in registers ran
+// slower, 0.555 ms on the 513x257 case); a particle is two 8-byte pairs
+// and vz (three accesses and addresses where five arrays take five); the
+// common chunk in which nothing leaves is stored where it was; and
+// movers are counted per destination by ballots over the code's four bits
+// (lane D holds code D's count; no shared-memory atomics).  vz is needed only
+// where the slot changes: a cell that had movers in the last step copies it
+// with the chunk, another one loads it when its first mover turns up (an
+// ion cell hardly ever has one: 4 of 36 bytes per particle past chunk 0).
+// Measured on a B200, five arrays and a ring of three chunks ahead against
+// this form: 0.532 and 0.487 ms on the 513x257 case with 200 particles per
+// cell and species, 0.219 and 0.204 ms with 20.
+constexpr int MOVE_MINB = 2;
+constexpr int MOVE_RING = 5;
+constexpr int MOVE_SLOT = 5 * 32; // floats per ring slot: (x, y), (vx, vy), vz
 
 template <int R>
-__global__ void __launch_bounds__(512) k_move(const DevCase *__restrict__ cases,
-                                                   const int *__restrict__ item_start, int ncases, int items) {
-    extern __shared__ float move_ring_s[];
-    __shared__ int dc_s[16][12]; // at most 16 warps per block (512 threads)
-    float *ring = move_ring_s + (threadIdx.x >> 5) * (R * 5 * 32);
-    int *dc = dc_s[threadIdx.x >> 5];
+__global__ void __launch_bounds__(512, MOVE_MINB) k_move(const DevCase *__restrict__ cases,
+                                                 const int *__restrict__ item_start, int ncases, int items) {
+    extern __shared__ __align__(16) float move_ring_s[];
+    float *const ring = move_ring_s + (threadIdx.x >> 5) * (R * MOVE_SLOT);
     const int warp = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if (warp >= items) return;
     const int ci = find_case(item_start, ncases, warp);
     const DevCase &d = cases[ci];
-    const int w = warp - item_start[ci];
-    const int s = w / d.C, c = w - s * d.C;
+    const unsigned w = (unsigned)(warp - item_start[ci]);
+    const int s = (int)d.div_c.quot(w), c = (int)w - s * d.C;
     const DevSpecies &sp = d.sp[s];
     const int cap = sp.cap;
     const size_t base = (size_t)c * cap;
-    const int i = c / d.ncy, j = c - i * d.ncy;
-    const int node = i * d.ngy + j;
-    // the count, the cell's field corners and the first chunk are independent
-    // loads: issue them together (slots 0..31 of a cell are always inside the
-    // pool, cap >= 32; lanes past the count are ignored)
-    const int n = sp.cnt[c];
-    const float ex_ws = d.Ex[node], ex_wn = d.Ex[node + 1], ex_es = d.Ex[node + d.ngy], ex_en = d.Ex[node + d.ngy + 1];
-    const float ey_ws = d.Ey[node], ey_wn = d.Ey[node + 1], ey_es = d.Ey[node + d.ngy], ey_en = d.Ey[node + d.ngy + 1];
-    // chunk q of the cell (all 32 slots: k0 + 32 <= cap, as cap is a multiple
-    // of 32 and k0 < n <= cap) goes to ring slot q % R as 16-byte copies: lanes
-    // 0-7 x, 8-15 y, 16-23 vx, 24-31 vy, then lanes 0-7 vz; one commit group
-    // per chunk (possibly empty)
-    const float *arr4 = lane < 8 ? sp.x : lane < 16 ? sp.y : lane < 24 ? sp.vx : sp.vy;
-    auto issue = [&](int k0, int lim) {
-        float *sl = ring + ((k0 >> 5) % R) * 160;
+    float2 *const xy = sp.xy + base, *const v = sp.v + base;
+    float *const vz = sp.vz + base;
+    // chunk q (all 32 slots are inside the cell: k0 < n <= cap, cap a multiple
+    // of 32) goes to ring slot q % R: lanes 0-15 copy (x, y), 16-31 (vx, vy), then
+    // lanes 0-7 vz where asked for; one commit group per chunk (possibly empty)
+    const float *const pair = (const float *)(lane < 16 ? xy : v) + 4 * (lane & 15);
+    auto issue = [&](int k0, int lim, bool with_z) {
+        float *sl = ring + ((k0 >> 5) % R) * MOVE_SLOT;
         if (k0 < lim) {
-            cp_async16(sl + 4 * lane, arr4 + base + k0 + 4 * (lane & 7));
-            if (lane < 8) cp_async16(sl + 128 + 4 * lane, sp.vz + base + k0 + 4 * lane);
+            cp_async16(sl + 4 * lane, pair + 2 * k0);
+            if (with_z && lane < 8) cp_async16(sl + 128 + 4 * lane, vz + k0 + 4 * lane);
         }
         cp_async_commit();
     };
-    issue(0, 32); // slots 0..31 of a cell are always inside the pool (cap >= 32)
-    // an interior cell whose 3x3 neighbourhood is all plasma (ghost code 0):
-    // a particle that ends in a neighbour after one wrap needs no walk
-    const int g3 = lane < 9 ? d.sidx[(i + lane / 3) * (d.ncy + 2) + (j + lane % 3)] : 0;
-    const bool open3 = __ballot_sync(FULL, g3 != 0) == 0u && i >= 1 && i + 1 < d.ncx && j >= 1 && j + 1 < d.ncy;
-    if (n == 0) {
-        cp_async_wait_all();
-        if (lane == 0) sp.nmov[c] = 0;
-        if (lane < 9) sp.dcount[(size_t)c * 9 + lane] = 0;
-        return;
-    }
-    if (lane == 0) atomicAdd(&d.pushes[warp & 31], (unsigned long long)n);
-    if (2 * n > cap) { // the reference's ReArg condition (src/cuda_Sortboundary.cu:63-65)
+    issue(0, 32, true); // slots 0..31 of a cell are always inside the pool (cap >= 32)
+    // the count, the cell's field corners and the first chunk are independent
+    // loads: issue them together
+    const int n = sp.cnt[c];
+    const int had = sp.nmov[c]; // movers of the last step
+    const int i = (int)d.div_ncy.quot((unsigned)c), j = c - i * d.ncy;
+    const int node = i * d.ngy + j;
+    const float ex_ws = d.Ex[node], ex_wn = d.Ex[node + 1], ex_es = d.Ex[node + d.ngy], ex_en = d.Ex[node + d.ngy + 1];
+    const float ey_ws = d.Ey[node], ey_wn = d.Ey[node + 1], ey_es = d.Ey[node + d.ngy], ey_en = d.Ey[node + d.ngy + 1];
+    const bool open3 = d.open3[c] != 0; // 3x3 neighbourhood all plasma: a one-wrap mover needs no walk
+    if (n == 0 || 2 * n > cap) {
         if (lane == 0) {
             sp.nmov[c] = 0;
-            atomicOr(d.status, ST_OVERFLOW);
+            if (n) { // the reference's ReArg condition (src/cuda_Sortboundary.cu:63-65)
+                atomicAdd(&d.pushes[warp & 31], (unsigned long long)n);
+                atomicOr(d.status, ST_OVERFLOW);
+            }
         }
         if (lane < 9) sp.dcount[(size_t)c * 9 + lane] = 0;
         cp_async_wait_all();
         return;
     }
+    int zfrom = had > 0 ? 0 : n; // chunks from here on, and chunk 0, come with vz
 #pragma unroll
-    for (int q = 1; q < R - 1; q++) issue(q * 32, n);
+    for (int q = 1; q < R - 1; q++) issue(q * 32, n, had > 0);
     const float As = sp.Ascale, dtdx = d.dt_dx, dtdy = d.dt_dy;
     const unsigned lt = lanemask_lt();
-    int m = 0, shifted = 0;
-    // movers per destination code, counted in shared memory
-    if (lane < 9) dc[lane] = 0;
-    __syncwarp();
-    // R - 1 chunks in flight while one is pushed (stores only go to slots at
-    // or below the current chunk, or to the top region at or above
-    // cap - n >= n, so no slot still to be copied is touched)
+    int m = 0, to_code = 0;
+    int first = n; // first slot that changes: the first mover's
+    // stores only go to slots at or below the current chunk, or to the top
+    // region at or above cap - n >= n, so no slot still to be loaded is touched
     for (int k0 = 0; k0 < n; k0 += 32) {
         const int k = k0 + lane;
         const bool act = k < n;
-        issue(k0 + (R - 1) * 32, n);
+        const int kn = k0 + (R - 1) * 32;
+        issue(kn, n, kn >= zfrom);
         cp_async_wait<R - 1>();
-        __syncwarp(); // the chunk was copied by eight lanes per array
-        const float *sl = ring + ((k0 >> 5) % R) * 160;
-        float lx = sl[lane], ly = sl[32 + lane], vx = sl[64 + lane], vy = sl[96 + lane];
-        const float vz = sl[128 + lane];
+        __syncwarp(); // the chunk was copied by other lanes
+        const float *const sl = ring + ((k0 >> 5) % R) * MOVE_SLOT;
+        const float2 pxy = ((const float2 *)sl)[lane], pv = ((const float2 *)sl)[32 + lane];
+        float lx = pxy.x, ly = pxy.y, mvX = pv.x, mvY = pv.y, z = 0.f;
         // bilinear weights once, then fused multiply-adds (one rounding each)
         const float wx = 1 - lx, wy = 1 - ly;
         const float w00 = wx * wy, w01 = wx * ly, w10 = lx * wy, w11 = lx * ly;
         const float del_vx = __fmaf_rn(ex_en, w11, __fmaf_rn(ex_es, w10, __fmaf_rn(ex_wn, w01, ex_ws * w00)));
         const float del_vy = __fmaf_rn(ey_en, w11, __fmaf_rn(ey_es, w10, __fmaf_rn(ey_wn, w01, ey_ws * w00)));
-        float mvX = __fmaf_rn(del_vx, As, vx);
-        float mvY = __fmaf_rn(del_vy, As, vy);
+        mvX = __fmaf_rn(del_vx, As, mvX);
+        mvY = __fmaf_rn(del_vy, As, mvY);
         lx = __fmaf_rn(mvX, dtdx, lx);
         ly = __fmaf_rn(mvY, dtdy, ly);
-        const bool out = act && (ly >= 1 || ly < 0 || lx >= 1 || lx < 0);
-        int code = 4, fi = i, fj = j;
-        bool near = false;
-        if (out && open3) { // the walk's first crossing with ghost code 0: a wrap, no flip
-            // (lx - (float)di is lx - 1, lx + 1 or lx, exactly the walk's wrap)
-            const int dj = (int)(ly >= 1) - (int)(ly < 0), di = (int)(lx >= 1) - (int)(lx < 0);
-            const float wy = ly - (float)dj, wx = lx - (float)di;
-            if (!(wy >= 1 || wy < 0 || wx >= 1 || wx < 0)) {
-                lx = wx;
-                ly = wy;
-                code = 3 * di + dj + 4;
-                near = true;
+        // bit patterns below that of 1 are exactly [+0, 1): anything else is
+        // looked at again (-0 and NaN stay, as the comparisons below say)
+        const bool odd = act && max(__float_as_uint(lx), __float_as_uint(ly)) >= 0x3f800000u;
+        if (__ballot_sync(FULL, odd) == 0u && m == 0) {
+            if (act) {
+                xy[k] = make_float2(lx, ly);
+                v[k] = make_float2(mvX, mvY);
             }
+            continue;
         }
-        if (out && !near) {
-            int cond = -1;
-            const int r = walk(geo_of(d), fi, fj, lx, ly, mvX, mvY, cond);
-            if (r) {
-                code = CODE_ABSORBED;
-                if (cond >= 0 && cond < d.cond_numr) {
-                    atomicAdd(&d.cond_charge[s * d.cond_numr + cond], 1.0f);
-                    if (d.cond_step) atomicAdd(&d.cond_step[s * d.cond_numr + cond], 1u);
-                } else if (cond <= -2 && d.sig) {
-                    surface_enqueue(d, s, fi, fj, -2 - cond, lx, ly, mvX, mvY);
+        const bool out = odd && (ly >= 1 || ly < 0 || lx >= 1 || lx < 0);
+        int code = 4, far_to = 0;
+        if (out) {
+            bool near = false;
+            if (open3) { // the walk's first crossing with ghost code 0: a wrap, no flip
+                // (subtracting +-1 or 0 is exactly the walk's wrap)
+                const float fy = ly >= 1 ? 1.f : ly < 0 ? -1.f : 0.f, fx = lx >= 1 ? 1.f : lx < 0 ? -1.f : 0.f;
+                const float ty = ly - fy, tx = lx - fx;
+                if (!(tx >= 1 || tx < 0 || ty >= 1 || ty < 0)) {
+                    code += (ly >= 1 ? 1 : ly < 0 ? -1 : 0) + (lx >= 1 ? 3 : lx < 0 ? -3 : 0);
+                    lx = tx;
+                    ly = ty;
+                    near = true;
                 }
-                if (r == 2) atomicOr(d.status, ST_WALK);
-            } else {
-                const int ddi = fi - i, ddj = fj - j;
-                code = (ddi >= -1 && ddi <= 1 && ddj >= -1 && ddj <= 1) ? (ddi + 1) * 3 + (ddj + 1) : CODE_FAR;
+            }
+            if (!near) {
+                const int ci = (int)d.div_ncy.quot((unsigned)c), cj = c - ci * d.ncy;
+                int fi = ci, fj = cj, cond = -1;
+                const int r = walk(geo_of(d), fi, fj, lx, ly, mvX, mvY, cond);
+                if (r) {
+                    code = CODE_ABSORBED;
+                    if (cond >= 0 && cond < d.cond_numr) {
+                        atomicAdd(&d.cond_charge[s * d.cond_numr + cond], 1.0f);
+                        if (d.cond_step) atomicAdd(&d.cond_step[s * d.cond_numr + cond], 1u);
+                    } else if (cond <= -2 && d.sig) {
+                        surface_enqueue(d, s, fi, fj, -2 - cond, lx, ly, mvX, mvY);
+                    }
+                    if (r == 2) atomicOr(d.status, ST_WALK);
+                } else {
+                    const int ddi = fi - ci, ddj = fj - cj;
+                    code = (ddi >= -1 && ddi <= 1 && ddj >= -1 && ddj <= 1) ? (ddi + 1) * 3 + (ddj + 1) : CODE_FAR;
+                    far_to = fi * d.ncy + fj;
+                }
             }
         }
-        if (out && code < 9) atomicAdd(&dc[code], 1);
         const unsigned bout = __ballot_sync(FULL, out);
+        if (bout) { // lane D < 9 counts the movers to code D: the lanes whose code bits equal D's
+            const unsigned b0 = __ballot_sync(FULL, code & 1), b1 = __ballot_sync(FULL, code & 2),
+                           b2 = __ballot_sync(FULL, code & 4), b3 = __ballot_sync(FULL, code & 8);
+            to_code += __popc(bout & ((lane & 1) ? b0 : ~b0) & ((lane & 2) ? b1 : ~b1) & ((lane & 4) ? b2 : ~b2) &
+                              ((lane & 8) ? b3 : ~b3));
+            if (m == 0) first = k0 + __ffs(bout) - 1;
+        }
         const int before = m + __popc(bout & lt);
         const bool moved = act && (out || before != 0); // its slot changes
-        shifted += __popc(__ballot_sync(FULL, moved));
+        if (moved) z = k0 == 0 || k0 >= zfrom ? sl[128 + lane] : vz[k];
+        if (zfrom == n && bout) zfrom = k0 + 32 * R;
         __syncwarp(); // every lane's loads of this chunk precede the in-place stores
         if (act) {
-            const size_t dst = out ? base + (size_t)(cap - 1 - before) : base + (size_t)(k - before);
-            sp.x[dst] = lx;
-            sp.y[dst] = ly;
-            sp.vx[dst] = mvX;
-            sp.vy[dst] = mvY;
-            if (moved) sp.vz[dst] = vz;
-            if (out) sp.code[dst] = (int8_t)code;
+            const int dst = out ? cap - 1 - before : k - before;
+            xy[dst] = make_float2(lx, ly);
+            v[dst] = make_float2(mvX, mvY);
+            if (moved) vz[dst] = z;
+            if (out) sp.code[base + dst] = (int8_t)code;
             if (code == CODE_FAR) {
-                const size_t b = (size_t)s * d.C + (size_t)(fi * d.ncy + fj);
+                const size_t b = (size_t)s * d.C + (size_t)far_to;
                 const int q = atomicAdd(&d.far_in[b], 1);
                 if (q < FAR_B)
                     d.far_key[b * FAR_B + q] = ((unsigned long long)c << 18) | (unsigned long long)before;
@@ -404,149 +421,11 @@ __global__ void __launch_bounds__(512) k_move(const DevCase *__restrict__ cases,
     if (lane == 0) {
         sp.cnt[c] = n - m;
         sp.nmov[c] = m;
-        atomicAdd(&d.pushes[32 + (warp & 31)], (unsigned long long)shifted);
+        atomicAdd(&d.pushes[warp & 31], (unsigned long long)n);
+        // every particle from the first mover on changed its slot
+        atomicAdd(&d.pushes[32 + (warp & 31)], (unsigned long long)(n - first));
     }
-    __syncwarp();
-    if (lane < 9) sp.dcount[(size_t)c * 9 + lane] = dc[lane];
-}
-
-// The same push with U chunks of 32 particles loaded per iteration before
-// any of them is pushed (5*U independent loads in flight per lane instead of
-// a one-chunk prefetch).  In-place stores of a chunk only reach slots at or
-// below it, and all U chunks are loaded before the first store of the
-// iteration, so no unread slot is overwritten.  Results, slot order, codes
-// and counts are identical to k_move's.
-template <int U>
-__global__ void __launch_bounds__(512) k_move_u(const DevCase *__restrict__ cases, const int *__restrict__ item_start,
-                                                int ncases, int items) {
-    const int warp = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
-    if (warp >= items) return;
-    const int ci = find_case(item_start, ncases, warp);
-    const DevCase &d = cases[ci];
-    const int w = warp - item_start[ci];
-    const int s = w / d.C, c = w - s * d.C;
-    const DevSpecies &sp = d.sp[s];
-    const int n = sp.cnt[c];
-    if (n == 0) {
-        if (lane == 0) sp.nmov[c] = 0;
-        if (lane < 9) sp.dcount[(size_t)c * 9 + lane] = 0;
-        return;
-    }
-    if (lane == 0) atomicAdd(&d.pushes[warp & 31], (unsigned long long)n);
-    const int cap = sp.cap;
-    if (2 * n > cap) { // the reference's ReArg condition (src/cuda_Sortboundary.cu:63-65)
-        if (lane == 0) {
-            sp.nmov[c] = 0;
-            atomicOr(d.status, ST_OVERFLOW);
-        }
-        if (lane < 9) sp.dcount[(size_t)c * 9 + lane] = 0;
-        return;
-    }
-    const int i = c / d.ncy, j = c - i * d.ncy;
-    const int node = i * d.ngy + j;
-    const float ex_ws = d.Ex[node], ex_wn = d.Ex[node + 1], ex_es = d.Ex[node + d.ngy], ex_en = d.Ex[node + d.ngy + 1];
-    const float ey_ws = d.Ey[node], ey_wn = d.Ey[node + 1], ey_es = d.Ey[node + d.ngy], ey_en = d.Ey[node + d.ngy + 1];
-    const float As = sp.Ascale, dtdx = d.dt_dx, dtdy = d.dt_dy;
-    const size_t base = (size_t)c * cap;
-    float *__restrict__ px = sp.x + base;
-    float *__restrict__ py = sp.y + base;
-    float *__restrict__ pvx = sp.vx + base;
-    float *__restrict__ pvy = sp.vy + base;
-    float *__restrict__ pvz = sp.vz + base;
-    const unsigned lt = lanemask_lt();
-    int m = 0, shifted = 0;
-    unsigned long long pk0 = 0, pk1 = 0, pk2 = 0;
-    for (int k0 = 0; k0 < n; k0 += 32 * U) {
-        float lx[U], ly[U], mvx[U], mvy[U], vz[U];
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const int k = k0 + 32 * u + lane;
-            lx[u] = ly[u] = mvx[u] = mvy[u] = vz[u] = 0.f;
-            if (k < n) {
-                lx[u] = px[k];
-                ly[u] = py[k];
-                mvx[u] = pvx[k];
-                mvy[u] = pvy[k];
-                vz[u] = pvz[k];
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const int k = k0 + 32 * u + lane;
-            const bool act = k < n;
-            const float x0 = lx[u], y0 = ly[u];
-            const float wx = 1 - x0, wy = 1 - y0;
-            const float w00 = wx * wy, w01 = wx * y0, w10 = x0 * wy, w11 = x0 * y0;
-            const float del_vx = __fmaf_rn(ex_en, w11, __fmaf_rn(ex_es, w10, __fmaf_rn(ex_wn, w01, ex_ws * w00)));
-            const float del_vy = __fmaf_rn(ey_en, w11, __fmaf_rn(ey_es, w10, __fmaf_rn(ey_wn, w01, ey_ws * w00)));
-            float vX = __fmaf_rn(del_vx, As, mvx[u]);
-            float vY = __fmaf_rn(del_vy, As, mvy[u]);
-            float X = __fmaf_rn(vX, dtdx, x0);
-            float Y = __fmaf_rn(vY, dtdy, y0);
-            const bool out = act && (Y >= 1 || Y < 0 || X >= 1 || X < 0);
-            int code = 4, fi = i, fj = j;
-            if (out) {
-                int cond = -1;
-                const int r = walk(geo_of(d), fi, fj, X, Y, vX, vY, cond);
-                if (r) {
-                    code = CODE_ABSORBED;
-                    if (cond >= 0 && cond < d.cond_numr) {
-                        atomicAdd(&d.cond_charge[s * d.cond_numr + cond], 1.0f);
-                        if (d.cond_step) atomicAdd(&d.cond_step[s * d.cond_numr + cond], 1u);
-                    } else if (cond <= -2 && d.sig) {
-                        surface_enqueue(d, s, fi, fj, -2 - cond, X, Y, vX, vY);
-                    }
-                    if (r == 2) atomicOr(d.status, ST_WALK);
-                } else {
-                    const int ddi = fi - i, ddj = fj - j;
-                    code = (ddi >= -1 && ddi <= 1 && ddj >= -1 && ddj <= 1) ? (ddi + 1) * 3 + (ddj + 1) : CODE_FAR;
-                }
-                if (code < 9) {
-                    const int q3 = code / 3;
-                    const unsigned long long one = 1ull << (21 * (code - 3 * q3));
-                    if (q3 == 0) pk0 += one;
-                    else if (q3 == 1) pk1 += one;
-                    else pk2 += one;
-                }
-            }
-            const unsigned bout = __ballot_sync(FULL, out);
-            const int before = m + __popc(bout & lt);
-            shifted += __popc(__ballot_sync(FULL, act && (out || before != 0)));
-            __syncwarp(); // every lane's loads of this iteration precede the in-place stores
-            if (act) {
-                const int dst = out ? cap - 1 - before : k - before;
-                px[dst] = X;
-                py[dst] = Y;
-                pvx[dst] = vX;
-                pvy[dst] = vY;
-                pvz[dst] = vz[u];
-                if (out) sp.code[base + dst] = (int8_t)code;
-                if (code == CODE_FAR) {
-                    const size_t b = (size_t)s * d.C + (size_t)(fi * d.ncy + fj);
-                    const int q = atomicAdd(&d.far_in[b], 1);
-                    if (q < FAR_B)
-                        d.far_key[b * FAR_B + q] = ((unsigned long long)c << 18) | (unsigned long long)before;
-                    else
-                        atomicOr(d.status, ST_OVERFLOW);
-                }
-            }
-            m += __popc(bout);
-        }
-    }
-    if (lane == 0) {
-        sp.cnt[c] = n - m;
-        sp.nmov[c] = m;
-        atomicAdd(&d.pushes[32 + (warp & 31)], (unsigned long long)shifted);
-    }
-    int mine = 0;
-#pragma unroll
-    for (int D = 0; D < 9; D++) {
-        const unsigned long long wv = D < 3 ? pk0 : D < 6 ? pk1 : pk2;
-        const unsigned tt = __reduce_add_sync(FULL, (unsigned)((wv >> (21 * (D % 3))) & 0x1FFFFFull));
-        if (lane == D) mine = (int)tt;
-    }
-    if (lane < 9) sp.dcount[(size_t)c * 9 + lane] = mine;
+    if (lane < 9) sp.dcount[(size_t)c * 9 + lane] = to_code;
 }
 
 // ------------------------------------------------------------------ Sort
@@ -574,7 +453,7 @@ constexpr int SORT_MAXW = 16; // warps per block, at most
 #ifndef SORT_PRE
 #define SORT_PRE 4
 #endif
-constexpr int SORT_SLOT = 5 * 32 + 8; // floats per ring slot: x, y, vx, vy, vz, then 32 code bytes
+constexpr int SORT_SLOT = 5 * 32 + 8; // floats per ring slot: (x, y), (vx, vy), vz, then 32 code bytes
 #ifndef SORT_MINB
 #define SORT_MINB 2 // resident blocks per SM the register budget is set for
 #endif
@@ -599,16 +478,16 @@ __global__ void __launch_bounds__(SORT_MAXW * 32, SORT_MINB) k_sort_push(const D
     // chunk h (movers 32h .. 32h+31) is the 32 slots cap-32-32h .. cap-1-32h,
     // all inside the cell as m <= cap/2 and cap is a multiple of 32; mover
     // 32h + l is element 31 - l of each array in ring slot h % SORT_PRE.
-    // Lanes 0-7 copy x, 8-15 y, 16-23 vx, 24-31 vy, then lanes 0-7 vz and
+    // Lanes 0-15 copy (x, y), 16-31 (vx, vy), then lanes 0-7 vz and
     // lanes 8-9 the codes; one commit group per chunk (possibly empty).  Slots
     // of the chunk below the movers belong to the cell's free region, which
     // other warps may be filling: those values are copied but never used
-    const float *arr4 = lane < 8 ? sp.x : lane < 16 ? sp.y : lane < 24 ? sp.vx : sp.vy;
+    const float *pair = (const float *)(lane < 16 ? sp.xy : sp.v);
     auto issue = [&](int h, bool any) {
         if (any) {
             float *sl = ring + (h % SORT_PRE) * SORT_SLOT;
             const size_t o = base + (size_t)(cap - 32 - 32 * h);
-            cp_async16(sl + 4 * lane, arr4 + o + 4 * (lane & 7));
+            cp_async16(sl + 4 * lane, pair + 2 * o + 4 * (lane & 15));
             if (lane < 8) cp_async16(sl + 128 + 4 * lane, sp.vz + o + 4 * lane);
             else if (lane < 10) cp_async16(sl + 160 + 4 * (lane - 8), (const float *)(sp.code + o) + 4 * (lane - 8));
         }
@@ -666,8 +545,8 @@ __global__ void __launch_bounds__(SORT_MAXW * 32, SORT_MINB) k_sort_push(const D
         __syncwarp(); // the chunk was copied by other lanes
         const float *sl = ring + (h % SORT_PRE) * SORT_SLOT;
         const int code = 32 * h + lane < m ? (int)((const int8_t *)(sl + 160))[31 - lane] : -1;
-        const float x = sl[31 - lane], y = sl[63 - lane], vx = sl[95 - lane], vy = sl[127 - lane],
-                    vz = sl[159 - lane];
+        const float2 xy = ((const float2 *)sl)[31 - lane], v = ((const float2 *)sl)[63 - lane];
+        const float vz = sl[159 - lane];
         __syncwarp(); // every lane has read the slot before it is refilled
         issue(h + SORT_PRE, 32 * (h + SORT_PRE) < m);
         // rank among this chunk's movers to the same destination (the lanes
@@ -683,10 +562,8 @@ __global__ void __launch_bounds__(SORT_MAXW * 32, SORT_MINB) k_sort_push(const D
         if (code >= 0 && code < 9) {
             if (slot < sm[code]) {
                 const size_t dst = (size_t)(c + (code / 3 - 1) * ncy + (code % 3 - 1)) * cap + (size_t)slot;
-                sp.x[dst] = x;
-                sp.y[dst] = y;
-                sp.vx[dst] = vx;
-                sp.vy[dst] = vy;
+                sp.xy[dst] = xy;
+                sp.v[dst] = v;
                 sp.vz[dst] = vz;
             } else {
                 overflow = true;
@@ -757,10 +634,8 @@ __global__ void __launch_bounds__(SORT_MAXW * 32) k_sort_count(const DevCase *__
                 const int sc = (int)(k8[t] >> 18), r = (int)(k8[t] & 0x3FFFF);
                 const size_t q = (size_t)sc * cap + (size_t)(cap - 1 - r);
                 const size_t dst = (size_t)c * cap + (size_t)slot;
-                sp.x[dst] = sp.x[q];
-                sp.y[dst] = sp.y[q];
-                sp.vx[dst] = sp.vx[q];
-                sp.vy[dst] = sp.vy[q];
+                sp.xy[dst] = sp.xy[q];
+                sp.v[dst] = sp.v[q];
                 sp.vz[dst] = sp.vz[q];
             } else {
                 overflow = true;
@@ -823,10 +698,8 @@ __global__ void __launch_bounds__(SORT_MAXW * 32) k_sort_count(const DevCase *__
                 const int sc = (int)(key[w] >> 18), r = (int)(key[w] & 0x3FFFF);
                 const size_t q = (size_t)sc * cap + (size_t)(cap - 1 - r);
                 const size_t dst = (size_t)fc * cap + (size_t)slot;
-                sp.x[dst] = sp.x[q];
-                sp.y[dst] = sp.y[q];
-                sp.vx[dst] = sp.vx[q];
-                sp.vy[dst] = sp.vy[q];
+                sp.xy[dst] = sp.xy[q];
+                sp.v[dst] = sp.v[q];
                 sp.vz[dst] = sp.vz[q];
             } else {
                 ov = true;
@@ -877,7 +750,8 @@ __device__ __forceinline__ int mcc_ion_collide(const DevCase &d, const DevSpecie
         const float b = hp_stream_next(&rs);
         maxwellv_dev(vnx, vny, vnz, d.vsave[nn], bvel, a, b);
     }
-    const float vx = ion.vx[q], vy = ion.vy[q], vz = ion.vz[q];
+    const float2 v = ion.v[q];
+    const float vx = v.x, vy = v.y, vz = ion.vz[q];
     float VX = vx - vnx, VY = vy - vnz, VZ = vz - vny; // y/z of the neutral swapped as in src/cuda_mccAr.cu:200-202
     const float dum = VX * VX + VY * VY + VZ * VZ;
     const float engy = ion.Escale * dum;
@@ -899,14 +773,14 @@ __device__ __forceinline__ int mcc_ion_collide(const DevCase &d, const DevSpecie
     } else {
         return -1; // velocity unchanged
     }
-    ion.vx[q] = ox;
-    ion.vy[q] = oy;
+    ion.v[q] = make_float2(ox, oy);
     ion.vz[q] = oz;
     return ch;
 }
 
 struct NewPair {
-    float x, y, evx, evy, evz, ivx, ivy, ivz;
+    float2 xy;
+    float evx, evy, evz, ivx, ivy, ivz;
 };
 
 // one electron that passed the null-collision test with draw R1; returns the
@@ -916,7 +790,8 @@ __device__ __forceinline__ int mcc_el_collide(const DevCase &d, const DevSpecies
                                               float R1, float P1, float bvel, NewPair &np) {
     int colltype = 1, ch = -1;
     const int target = (R1 <= P1) ? 0 : 1;
-    float VX = el.vx[q], VY = el.vy[q], VZ = el.vz[q];
+    const float2 v = el.v[q];
+    float VX = v.x, VY = v.y, VZ = el.vz[q];
     const float dum = VX * VX + VY * VY + VZ * VZ;
     float vel = sqrtf(dum);
     VX /= vel; VY /= vel; VZ /= vel;
@@ -958,8 +833,7 @@ __device__ __forceinline__ int mcc_el_collide(const DevCase &d, const DevSpecies
         engy -= rengy;
         vel = sqrtf(fabsf(rengy) / el.Escale);
         vel2 = sqrtf(fabsf(engy) / el.Escale);
-        np.x = el.x[q];
-        np.y = el.y[q];
+        np.xy = el.xy[q];
         np.evx = VX; np.evy = VY; np.evz = VZ;
         {
             const float a = hp_stream_next(&rs);
@@ -978,8 +852,7 @@ __device__ __forceinline__ int mcc_el_collide(const DevCase &d, const DevSpecies
     const float a = hp_stream_next(&rs);
     const float b = hp_stream_next(&rs);
     anewvel_dev(engy, vel, VX, VY, VZ, a, b);
-    el.vx[q] = VX;
-    el.vy[q] = VY;
+    el.v[q] = make_float2(VX, VY);
     el.vz[q] = VZ;
     return ch;
 }
@@ -1090,10 +963,12 @@ __device__ __forceinline__ void mcc_ar_cells(const DevCase &d, int c0, int n, in
                 const int se = m.ne + off, sn = m.ni + off;
                 if (se < el.cap && sn < ion.cap) {
                     const size_t qe = (size_t)m.c * el.cap + se, qi = (size_t)m.c * ion.cap + sn;
-                    el.x[qe] = np.x; el.y[qe] = np.y;
-                    el.vx[qe] = np.evx; el.vy[qe] = np.evy; el.vz[qe] = np.evz;
-                    ion.x[qi] = np.x; ion.y[qi] = np.y;
-                    ion.vx[qi] = np.ivx; ion.vy[qi] = np.ivy; ion.vz[qi] = np.ivz;
+                    el.xy[qe] = np.xy;
+                    el.v[qe] = make_float2(np.evx, np.evy);
+                    el.vz[qe] = np.evz;
+                    ion.xy[qi] = np.xy;
+                    ion.v[qi] = make_float2(np.ivx, np.ivy);
+                    ion.vz[qi] = np.ivz;
                 } else {
                     overflow = true;
                 }
@@ -1189,7 +1064,7 @@ __global__ void __launch_bounds__(512) k_deposit_cells(const DevCase *__restrict
     const int lane = threadIdx.x & 31;
     if (warp * G >= items) return;
     int my_n = 0;
-    const float *my_x = nullptr, *my_y = nullptr;
+    const float2 *my_xy = nullptr;
     double4 *my_cw = nullptr;
     if (lane < G && warp * G + lane < items) {
         const int item = warp * G + lane;
@@ -1200,28 +1075,25 @@ __global__ void __launch_bounds__(512) k_deposit_cells(const DevCase *__restrict
         const DevSpecies &sp = d.sp[s];
         const size_t base = (size_t)c * sp.cap;
         my_n = sp.cnt[c];
-        my_x = sp.x + base;
-        my_y = sp.y + base;
+        my_xy = sp.xy + base;
         my_cw = d.cw[s] + c;
     }
     int n[G];
-    const float *px[G], *py[G];
-    float x0[G], y0[G];
+    const float2 *pxy[G];
+    float2 f0[G];
 #pragma unroll
     for (int g = 0; g < G; g++) {
         n[g] = __shfl_sync(FULL, my_n, g);
-        px[g] = (const float *)__shfl_sync(FULL, (unsigned long long)my_x, g);
-        py[g] = (const float *)__shfl_sync(FULL, (unsigned long long)my_y, g);
+        pxy[g] = (const float2 *)__shfl_sync(FULL, (unsigned long long)my_xy, g);
     }
     // the first chunk of every cell: slots 0..31 are inside the pool (cap >= 32)
 #pragma unroll
     for (int g = 0; g < G; g++) {
-        x0[g] = px[g] ? px[g][lane] : 0.f;
-        y0[g] = py[g] ? py[g][lane] : 0.f;
+        f0[g] = pxy[g] ? pxy[g][lane] : make_float2(0.f, 0.f);
     }
 #pragma unroll
     for (int g = 0; g < G; g++) {
-        if (!px[g]) continue; // past the last item (warp-uniform)
+        if (!pxy[g]) continue; // past the last item (warp-uniform)
         const int ng = n[g];
         if (ng == 0) { // warp-uniform: the sums of an empty cell are +0, as the tree would give
             double4 *cw = (double4 *)__shfl_sync(FULL, (unsigned long long)my_cw, g);
@@ -1235,18 +1107,17 @@ __global__ void __launch_bounds__(512) k_deposit_cells(const DevCase *__restrict
             ES += lx * (1 - ly);
             EN += lx * ly;
         };
-        if (lane < ng) add(x0[g], y0[g]);
+        if (lane < ng) add(f0[g].x, f0[g].y);
         for (int k0 = 32; k0 < ng; k0 += 128) {
-            float xs[4], ys[4];
+            float2 f[4];
 #pragma unroll
             for (int h = 0; h < 4; h++) {
                 const int k = k0 + 32 * h + lane;
-                xs[h] = k < ng ? px[g][k] : 0.f;
-                ys[h] = k < ng ? py[g][k] : 0.f;
+                f[h] = k < ng ? pxy[g][k] : make_float2(0.f, 0.f);
             }
 #pragma unroll
             for (int h = 0; h < 4; h++)
-                if (k0 + 32 * h + lane < ng) add(xs[h], ys[h]);
+                if (k0 + 32 * h + lane < ng) add(f[h].x, f[h].y);
         }
         const double a = warp_sum_d(WS), b = warp_sum_d(WN), e = warp_sum_d(ES), f = warp_sum_d(EN);
         double4 *cw = (double4 *)__shfl_sync(FULL, (unsigned long long)my_cw, g);
@@ -2077,7 +1948,8 @@ __global__ void __launch_bounds__(256) k_eedf(const DevCase *__restrict__ cases,
             const int n = el.cnt[c];
             const size_t base = (size_t)c * el.cap;
             for (int k = lane; k < n; k += 32) {
-                const float vx = el.vx[base + k], vy = el.vy[base + k], vz = el.vz[base + k];
+                const float2 v = el.v[base + k];
+                const float vx = v.x, vy = v.y, vz = el.vz[base + k];
                 const float e = el.Escale * (vx * vx + vy * vy + vz * vz);
                 const int b = e < HP_EEDF_BINS * HP_EEDF_DE ? (int)(e * (1.0f / HP_EEDF_DE)) : HP_EEDF_BINS;
                 if (ci == case_of_block) atomicAdd(&h[b], 1u);
@@ -2104,10 +1976,8 @@ __global__ void __launch_bounds__(256) k_scatter(DevSpecies sp, int C, const int
     const size_t total = (size_t)start[C];
     const size_t base = (size_t)warp * sp.cap;
     for (int k = lane; k < n; k += 32) {
-        sp.x[base + k] = src[b + k];
-        sp.y[base + k] = src[total + b + k];
-        sp.vx[base + k] = src[2 * total + b + k];
-        sp.vy[base + k] = src[3 * total + b + k];
+        sp.xy[base + k] = make_float2(src[b + k], src[total + b + k]);
+        sp.v[base + k] = make_float2(src[2 * total + b + k], src[3 * total + b + k]);
         sp.vz[base + k] = src[4 * total + b + k];
     }
     if (lane == 0) {
@@ -2126,10 +1996,10 @@ cudaError_t launch_move(const DevCase *cases, const int *item_start, int ncases,
     const int tpb = 32 * std::min(std::max(lc.warps_per_block, 1), 16);
     const unsigned nb = blocks_for((long long)items * 32, tpb);
     prof::mark(st, "k_move");
-    if (lc.move_unroll == 2) k_move_u<2><<<nb, tpb, 0, st>>>(cases, item_start, ncases, items);
-    else if (lc.move_unroll == 4) k_move_u<4><<<nb, tpb, 0, st>>>(cases, item_start, ncases, items);
-    else
-        k_move<MOVE_RING><<<nb, tpb, (size_t)(tpb / 32) * MOVE_RING * 5 * 32 * sizeof(float), st>>>(cases, item_start, ncases, items);
+    const size_t slot = (size_t)(tpb / 32) * MOVE_SLOT * sizeof(float);
+    if (lc.move_unroll == 2) k_move<MOVE_RING - 1><<<nb, tpb, (MOVE_RING - 1) * slot, st>>>(cases, item_start, ncases, items);
+    else if (lc.move_unroll == 4) k_move<MOVE_RING + 2><<<nb, tpb, (MOVE_RING + 2) * slot, st>>>(cases, item_start, ncases, items);
+    else k_move<MOVE_RING><<<nb, tpb, MOVE_RING * slot, st>>>(cases, item_start, ncases, items);
     return cudaGetLastError();
 }
 

@@ -161,10 +161,8 @@ __global__ void k_load_place(PlaceArgs a) {
         slot = a.eslot[lo];
     }
     const size_t q = (size_t)D * a.sp.cap + (size_t)slot;
-    a.sp.x[q] = a.tmp[k];
-    a.sp.y[q] = a.tmp[a.np + k];
-    a.sp.vx[q] = a.tmp[2 * a.np + k];
-    a.sp.vy[q] = a.tmp[3 * a.np + k];
+    a.sp.xy[q] = make_float2(a.tmp[k], a.tmp[a.np + k]);
+    a.sp.v[q] = make_float2(a.tmp[2 * a.np + k], a.tmp[3 * a.np + k]);
     a.sp.vz[q] = a.tmp[4 * a.np + k];
 }
 

@@ -563,22 +563,23 @@ __device__ __forceinline__ void mcc_oxy_cells(const DevCase &d, int c0, int ncel
                 q = ent >> 24;
                 const int c = cs[q].c;
                 const size_t base = (size_t)c * sp.cap;
-                px = sp.x[base + k];
+                const float2 at = sp.xy[base + k];
+                px = at.x;
                 if (!is_hole(px)) { // an O- removed earlier this call is gone
                     active = true;
-                    py = sp.y[base + k];
-                    const float vx = sp.vx[base + k], vy = sp.vy[base + k], vz = sp.vz[base + k];
+                    py = at.y;
+                    const float2 v = sp.v[base + k];
+                    const float vx = v.x, vy = v.y, vz = sp.vz[base + k];
                     hp_stream rs;
                     hp_stream_init(&rs, d.seed, (uint32_t)k, (uint32_t)c, step, (uint32_t)s);
                     if (s == 0) electron_collide<GAS>(d, vx, vy, vz, t, cs[q].bv1, rs, o);
                     else ion_collide<GAS>(d, s, vx, vy, vz, t, cs[q].bv1, cs[q].bv2, rs, o);
                     if (o.ch >= 0) atomicAdd(&d.mcc_count[(size_t)c * d.mcc_stride + o.ch], 1u);
                     if (o.keep) {
-                        sp.vx[base + k] = o.vx;
-                        sp.vy[base + k] = o.vy;
+                        sp.v[base + k] = make_float2(o.vx, o.vy);
                         sp.vz[base + k] = o.vz;
                     } else {
-                        sp.x[base + k] = __int_as_float(0x7fc00000); // hole
+                        sp.xy[base + k].x = __int_as_float(0x7fc00000); // hole
                     }
                 }
             }
@@ -601,10 +602,8 @@ __device__ __forceinline__ void mcc_oxy_cells(const DevCase &d, int c0, int ncel
                     const int slot = cs[q].cnt[t] + __popc(bm & same & lt);
                     if (slot < tp.cap) {
                         const size_t q2 = (size_t)cs[q].c * tp.cap + slot;
-                        tp.x[q2] = px;
-                        tp.y[q2] = py;
-                        tp.vx[q2] = o.b[b].vx;
-                        tp.vy[q2] = o.b[b].vy;
+                        tp.xy[q2] = make_float2(px, py);
+                        tp.v[q2] = make_float2(o.b[b].vx, o.b[b].vy);
                         tp.vz[q2] = o.b[b].vz;
                     } else {
                         overflow = true;
@@ -628,7 +627,7 @@ __device__ __forceinline__ void mcc_oxy_cells(const DevCase &d, int c0, int ncel
                 int victim = -1;
                 if (lane == 0) {
                     int nlive = 0;
-                    for (int a = 0; a < nom; a++) nlive += is_hole(om.x[ob + a]) ? 0 : 1;
+                    for (int a = 0; a < nom; a++) nlive += is_hole(om.xy[ob + a].x) ? 0 : 1;
                     if (nlive > 0) {
                         int pick = 0;
                         if (nlive > 1) {
@@ -636,10 +635,10 @@ __device__ __forceinline__ void mcc_oxy_cells(const DevCase &d, int c0, int ncel
                             if (pick > nlive - 1) pick = nlive - 1;
                         }
                         for (int a = 0; a < nom; a++) {
-                            if (is_hole(om.x[ob + a])) continue;
+                            if (is_hole(om.xy[ob + a].x)) continue;
                             if (pick-- == 0) { victim = a; break; }
                         }
-                        om.x[ob + victim] = __int_as_float(0x7fc00000);
+                        om.xy[ob + victim].x = __int_as_float(0x7fc00000);
                     }
                 }
                 victim = __shfl_sync(FULL, victim, 0);
@@ -708,15 +707,16 @@ __device__ __forceinline__ void mcc_oxy_cells(const DevCase &d, int c0, int ncel
                         h[b + 1] = v;
                     }
                     for (int a = 0; a < nh; a++) {
-                        while (n > 0 && is_hole(sp.x[base + n - 1])) n--;
+                        while (n > 0 && is_hole(sp.xy[base + n - 1].x)) n--;
                         const int hpos = h[a];
                         if (hpos >= n) continue;
                         const size_t from = base + n - 1, to = base + hpos;
-                        sp.x[to] = sp.x[from]; sp.y[to] = sp.y[from];
-                        sp.vx[to] = sp.vx[from]; sp.vy[to] = sp.vy[from]; sp.vz[to] = sp.vz[from];
+                        sp.xy[to] = sp.xy[from];
+                        sp.v[to] = sp.v[from];
+                        sp.vz[to] = sp.vz[from];
                         n--;
                     }
-                    while (n > 0 && is_hole(sp.x[base + n - 1])) n--;
+                    while (n > 0 && is_hole(sp.xy[base + n - 1].x)) n--;
                     sp.cnt[c] = n;
                 }
             } else {
@@ -724,15 +724,18 @@ __device__ __forceinline__ void mcc_oxy_cells(const DevCase &d, int c0, int ncel
                 int out = 0;
                 for (int k0 = 0; k0 < n; k0 += 32) {
                     const int k = k0 + lane;
-                    float x = 0.f, y = 0.f, vx = 0.f, vy = 0.f, vz = 0.f;
+                    float2 xy = make_float2(0.f, 0.f), v = xy;
+                    float vz = 0.f;
                     const bool in = k < n;
-                    if (in) { x = sp.x[base + k]; y = sp.y[base + k]; vx = sp.vx[base + k]; vy = sp.vy[base + k]; vz = sp.vz[base + k]; }
-                    const bool live = in && !is_hole(x);
+                    if (in) { xy = sp.xy[base + k]; v = sp.v[base + k]; vz = sp.vz[base + k]; }
+                    const bool live = in && !is_hole(xy.x);
                     const unsigned bl = __ballot_sync(FULL, live);
                     __syncwarp();
                     if (live) {
                         const size_t to = base + out + __popc(bl & lt);
-                        sp.x[to] = x; sp.y[to] = y; sp.vx[to] = vx; sp.vy[to] = vy; sp.vz[to] = vz;
+                        sp.xy[to] = xy;
+                        sp.v[to] = v;
+                        sp.vz[to] = vz;
                     }
                     out += __popc(bl);
                     __syncwarp();

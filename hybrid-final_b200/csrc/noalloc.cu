@@ -45,7 +45,8 @@ __global__ void __launch_bounds__(256) k_na_cells(const hp::DevCase *__restrict_
     const size_t base = (size_t)c * sp.cap;
     float WS = 0.f, WN = 0.f, ES = 0.f, EN = 0.f;
     for (int k = lane; k < n; k += 32) {
-        const float lx = sp.x[base + k], ly = sp.y[base + k];
+        const float2 f = sp.xy[base + k];
+        const float lx = f.x, ly = f.y;
         WS += (1 - lx) * (1 - ly);
         WN += (1 - lx) * ly;
         ES += lx * (1 - ly);
