@@ -436,150 +436,173 @@ __global__ void __launch_bounds__(512, MOVE_MINB) k_move(const DevCase *__restri
 // cell index and each source's movers in list order, then the movers that
 // travelled further (its bucket) in (source cell, r) order.  The boundary
 // rules were applied by Move, which also counted each cell's movers per
-// destination (dcount).  From those counts every source knows where its
-// movers go, so the re-binning is a push with no loop-carried dependency:
-//   k_sort_push  (warp per source cell) slot of each near mover = stayers of
-//                the destination + movers sent to it by lower-index sources
-//                + rank among this source's movers to it;
-//   k_sort_count (lane per destination cell) new count, then the far movers.
+// destination (dcount).  Two passes, no loop-carried dependency in either:
+//   k_sort_count  (lane per destination cell) runs over the nine counts
+//                addressed to it in source order, puts in the place of each
+//                the slot that source's movers start at, finishes the far
+//                movers and writes the new count;
+//   k_sort_push  (warp per source cells) puts each near mover at its start
+//                slot + its rank among the source's movers to that cell.
+// A (source, code) count is addressed to one cell, so the plan replaces it in
+// place, and a source finds the nine slots it needs side by side.  (Summing
+// the counts of the lower-index sources in the push instead takes 81 loads and
+// index computations per source cell.)
 constexpr int SORT_MAXW = 16; // warps per block, at most
 
-// Memory-level parallelism: a source warp's movers arrive through a ring of
-// SORT_PRE chunk slots in shared memory, filled by asynchronous 16-byte copies
-// of the cell's top slots (no registers held while they are in flight); the
-// first chunk is requested before the mover count is known (the top 32 slots
-// exist in every cell), the next ones with the destinations' counts, so a
-// warp waits for about one round trip after its count.
-#ifndef SORT_PRE
-#define SORT_PRE 4
-#endif
+constexpr int SORT_MINB = 2; // resident 512-thread blocks per SM the register budget is set for
+constexpr int SORT_PRE = 4; // ring slots per warp: chunks of 32 movers in flight
+constexpr int SORT_G = 4; // items per warp, at most
 constexpr int SORT_SLOT = 5 * 32 + 8; // floats per ring slot: (x, y), (vx, vy), vz, then 32 code bytes
-#ifndef SORT_MINB
-#define SORT_MINB 2 // resident blocks per SM the register budget is set for
-#endif
 
-// One warp per (species, source cell): its movers (the r-th at slot cap-1-r)
-// go to their destinations' free slots in (source, rank) order.
+// Movers (the r-th at slot cap-1-r) to their destinations' free slots.  The
+// kernel is bound by memory latency and the sectors its stores touch, not by
+// instructions.  A warp takes up to SORT_G consecutive (species, cell) items
+// and reads their mover counts at once, so that cells without movers (nearly
+// all of an ion species') cost one load per group; the movers of the others
+// form one stream of chunks of 32, copied asynchronously into a ring of
+// SORT_PRE slots per warp in shared memory, across the borders of the cells.
+// The nine start slots, limits and cells of a cell are held by lanes 0-8
+// and loaded one cell ahead; a mover's rank comes from ballots over the
+// code's four bits.
+// Measured on a B200, one cell per warp that sums the lower-index sources'
+// counts itself against this form: 0.247 and 0.240 ms on the 513x257 case with 200
+// particles per cell and species, 0.132 and 0.069 ms with 20, 0.081 and 0.048 ms
+// on the 257x129 Ar/O2 case.
 __global__ void __launch_bounds__(SORT_MAXW * 32, SORT_MINB) k_sort_push(const DevCase *__restrict__ cases,
-                                                           const int *__restrict__ item_start, int ncases, int items) {
-    extern __shared__ float sort_ring_s[];
-    __shared__ int s_off[SORT_MAXW][9], s_lim[SORT_MAXW][9];
+                                                           const int *__restrict__ item_start, int ncases, int items,
+                                                           int per_warp) {
+    extern __shared__ __align__(16) float sort_ring_s[];
     const int warp = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-    if (warp >= items) return;
-    float *ring = sort_ring_s + wl * (SORT_PRE * SORT_SLOT);
-    const int ci = find_case(item_start, ncases, warp);
-    const DevCase &d = cases[ci];
-    const int w = warp - item_start[ci];
-    const int s = w / d.C, c = w - s * d.C;
-    const DevSpecies &sp = d.sp[s];
-    const int cap = sp.cap, ncy = d.ncy;
-    const size_t base = (size_t)c * cap;
-    // chunk h (movers 32h .. 32h+31) is the 32 slots cap-32-32h .. cap-1-32h,
-    // all inside the cell as m <= cap/2 and cap is a multiple of 32; mover
-    // 32h + l is element 31 - l of each array in ring slot h % SORT_PRE.
-    // Lanes 0-15 copy (x, y), 16-31 (vx, vy), then lanes 0-7 vz and
-    // lanes 8-9 the codes; one commit group per chunk (possibly empty).  Slots
-    // of the chunk below the movers belong to the cell's free region, which
-    // other warps may be filling: those values are copied but never used
-    const float *pair = (const float *)(lane < 16 ? sp.xy : sp.v);
-    auto issue = [&](int h, bool any) {
-        if (any) {
-            float *sl = ring + (h % SORT_PRE) * SORT_SLOT;
-            const size_t o = base + (size_t)(cap - 32 - 32 * h);
-            cp_async16(sl + 4 * lane, pair + 2 * o + 4 * (lane & 15));
-            if (lane < 8) cp_async16(sl + 128 + 4 * lane, sp.vz + o + 4 * lane);
-            else if (lane < 10) cp_async16(sl + 160 + 4 * (lane - 8), (const float *)(sp.code + o) + 4 * (lane - 8));
-        }
-        cp_async_commit();
+    const int lane = threadIdx.x & 31;
+    float *const ring = sort_ring_s + (threadIdx.x >> 5) * (SORT_PRE * SORT_SLOT);
+    const long long item0 = (long long)warp * per_warp;
+    if (item0 >= items) return;
+    // lane q holds item q: where it is, its movers, and the 32 top slots of its arrays
+    int my_case = 0, my_s = 0, my_c = 0, my_m = 0;
+    const float2 *my_xy = nullptr, *my_v = nullptr;
+    const float *my_vz = nullptr;
+    const int8_t *my_code = nullptr;
+    if (lane < per_warp && item0 + lane < items) {
+        const int item = (int)item0 + lane;
+        my_case = find_case(item_start, ncases, item);
+        const DevCase &d = cases[my_case];
+        const unsigned w = (unsigned)(item - item_start[my_case]);
+        my_s = (int)d.div_c.quot(w);
+        my_c = (int)w - my_s * d.C;
+        const DevSpecies &sp = d.sp[my_s];
+        const size_t top = (size_t)my_c * sp.cap + (size_t)(sp.cap - 32);
+        my_m = sp.nmov[my_c];
+        my_xy = sp.xy + top;
+        my_v = sp.v + top;
+        my_vz = sp.vz + top;
+        my_code = sp.code + top;
+    }
+    unsigned todo = __ballot_sync(FULL, my_m > 0), ahead = todo;
+    if (!todo) return;
+    auto shfl_ptr = [&](const void *p, int src) {
+        return (const float *)__shfl_sync(FULL, (unsigned long long)p, src);
     };
-    issue(0, true);
-    const int m = sp.nmov[c];
-    if (m == 0) {
-        cp_async_wait_all();
-        return;
-    }
-#pragma unroll
-    for (int h = 1; h < SORT_PRE; h++) issue(h, 32 * h < m);
-    const int i = c / ncy, j = c - i * ncy;
-    // destination D = code (di+1)*3 + (dj+1): its stayers and slot limit ...
-    int off9 = 0, lim9 = 0;
-    if (lane < 9) {
-        const int Di = i + lane / 3 - 1, Dj = j + lane % 3 - 1;
-        if (Di >= 0 && Di < d.ncx && Dj >= 0 && Dj < ncy) {
-            const int D = Di * ncy + Dj;
-            off9 = sp.cnt[D];
-            lim9 = cap - sp.nmov[D];
-        }
-    }
-    // ... and the movers sent to D by its other neighbours S < c; (D, S) pair
-    // p = 9*Dd + Ss, S = D + (Ss/3 - 1, Ss%3 - 1), and S's code for D is 8 - Ss
-    int pv[3];
-#pragma unroll
-    for (int t = 0; t < 3; t++) {
-        const int p = lane + 32 * t;
-        pv[t] = 0;
-        if (p < 81) {
-            const int Dd = p / 9, Ss = p - 9 * Dd;
-            const int Di = i + Dd / 3 - 1, Dj = j + Dd % 3 - 1;
-            const int Si = Di + Ss / 3 - 1, Sj = Dj + Ss % 3 - 1;
-            const int S = Si * ncy + Sj;
-            if (Di >= 0 && Di < d.ncx && Dj >= 0 && Dj < ncy && Si >= 0 && Si < d.ncx && Sj >= 0 && Sj < ncy && S < c)
-                pv[t] = sp.dcount[(size_t)S * 9 + (8 - Ss)];
-        }
-    }
-    int *so = s_off[wl], *sm = s_lim[wl];
-    if (lane < 9) {
-        so[lane] = off9;
-        sm[lane] = lim9;
-    }
-    __syncwarp();
-#pragma unroll
-    for (int t = 0; t < 3; t++)
-        if (pv[t]) atomicAdd(&so[(lane + 32 * t) / 9], pv[t]);
-    __syncwarp();
-    const unsigned lt = lanemask_lt();
-    bool overflow = false;
-    for (int h = 0; 32 * h < m; h++) {
-        cp_async_wait<SORT_PRE - 1>();
-        __syncwarp(); // the chunk was copied by other lanes
-        const float *sl = ring + (h % SORT_PRE) * SORT_SLOT;
-        const int code = 32 * h + lane < m ? (int)((const int8_t *)(sl + 160))[31 - lane] : -1;
-        const float2 xy = ((const float2 *)sl)[31 - lane], v = ((const float2 *)sl)[63 - lane];
-        const float vz = sl[159 - lane];
-        __syncwarp(); // every lane has read the slot before it is refilled
-        issue(h + SORT_PRE, 32 * (h + SORT_PRE) < m);
-        // rank among this chunk's movers to the same destination (the lanes
-        // holding the same code); so[D] then advances by their number, added
-        // by the group's highest lane
-        const unsigned grp = __match_any_sync(FULL, code);
-        const int rank = __popc(grp & lt);
-        const bool near = code >= 0 && code < 9;
-        const int slot = near ? so[code] + rank : 0;
-        __syncwarp();
-        if (near && (grp >> lane) == 1u) so[code] += __popc(grp);
-        __syncwarp();
-        if (code >= 0 && code < 9) {
-            if (slot < sm[code]) {
-                const size_t dst = (size_t)(c + (code / 3 - 1) * ncy + (code % 3 - 1)) * cap + (size_t)slot;
-                sp.xy[dst] = xy;
-                sp.v[dst] = v;
-                sp.vz[dst] = vz;
-            } else {
-                overflow = true;
+    // The next chunk of the stream, chunk ih of item `ahead`: movers 32 ih ..
+    // 32 ih + 31 are the 32 slots that end 32 ih below the top, all inside the
+    // cell as m <= cap/2 and cap is a multiple of 32; mover 32 ih + l is element
+    // 31 - l.  Lanes 0-15 copy (x, y), 16-31 (vx, vy), then lanes 0-7 vz and
+    // lanes 8-9 the codes; one commit group per chunk (possibly empty).  Slots
+    // below the movers belong to the cell's free region, which other warps may be
+    // filling: those values are copied but never used.
+    int ih = 0, issued = 0;
+    auto issue = [&]() {
+        if (ahead) {
+            const int src = __ffs(ahead) - 1;
+            const float *const pxy = shfl_ptr(my_xy, src), *const pv = shfl_ptr(my_v, src);
+            const float *const pz = shfl_ptr(my_vz, src), *const pc = shfl_ptr(my_code, src);
+            const int m = __shfl_sync(FULL, my_m, src);
+            float *const sl = ring + (issued % SORT_PRE) * SORT_SLOT;
+            cp_async16(sl + 4 * lane, (lane < 16 ? pxy : pv) - 64 * ih + 4 * (lane & 15));
+            if (lane < 8) cp_async16(sl + 128 + 4 * lane, pz - 32 * ih + 4 * lane);
+            else if (lane < 10) cp_async16(sl + 128 + 4 * lane, pc - 8 * ih + 4 * (lane - 8));
+            if (32 * ++ih >= m) {
+                ih = 0;
+                ahead &= ahead - 1;
             }
         }
+        issued++;
+        cp_async_commit();
+    };
+    // lane q < 9: destination of code q (the cell (q/3 - 1, q%3 - 1) away), its
+    // first free slot for this source and its slot limit
+    auto destinations = [&](int src, int &D, int &at, int &lim) {
+        const DevCase &d = cases[__shfl_sync(FULL, my_case, src)];
+        const DevSpecies &sp = d.sp[__shfl_sync(FULL, my_s, src)];
+        const int c = __shfl_sync(FULL, my_c, src), ncy = d.ncy;
+        D = at = lim = 0;
+        if (lane < 9) {
+            const int i = (int)d.div_ncy.quot((unsigned)c), j = c - i * ncy;
+            const int Di = i + lane / 3 - 1, Dj = j + lane % 3 - 1;
+            if (Di >= 0 && Di < d.ncx && Dj >= 0 && Dj < ncy) {
+                D = Di * ncy + Dj;
+                at = sp.dcount[(size_t)c * 9 + lane];
+                lim = sp.cap - sp.nmov[D];
+            }
+        }
+    };
+#pragma unroll
+    for (int q = 0; q < SORT_PRE - 1; q++) issue();
+    const unsigned lt = lanemask_lt();
+    int nD, nat, nlim, done = 0;
+    destinations(__ffs(todo) - 1, nD, nat, nlim);
+    while (todo) {
+        const int src = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const int D = nD, lim = nlim;
+        int at = nat;
+        if (todo) destinations(__ffs(todo) - 1, nD, nat, nlim);
+        const DevCase &d = cases[__shfl_sync(FULL, my_case, src)];
+        const DevSpecies &sp = d.sp[__shfl_sync(FULL, my_s, src)];
+        const int m = __shfl_sync(FULL, my_m, src), cap = sp.cap;
+        float2 *const oxy = sp.xy, *const ov = sp.v;
+        float *const oz = sp.vz;
+        bool overflow = false;
+        for (int h = 0; 32 * h < m; h++) {
+            issue();
+            cp_async_wait<SORT_PRE - 1>();
+            __syncwarp(); // the chunk was copied by other lanes
+            const float *const sl = ring + (done++ % SORT_PRE) * SORT_SLOT;
+            const float2 xy = ((const float2 *)sl)[31 - lane], v = ((const float2 *)sl)[63 - lane];
+            const float vz = sl[159 - lane];
+            const int code = (int)((const int8_t *)(sl + 160))[31 - lane];
+            __syncwarp(); // every lane has read the slot before it is refilled
+            const bool near = 32 * h + lane < m && code < 9;
+            const unsigned bn = __ballot_sync(FULL, near);
+            const unsigned b0 = __ballot_sync(FULL, code & 1), b1 = __ballot_sync(FULL, code & 2),
+                           b2 = __ballot_sync(FULL, code & 4), b3 = __ballot_sync(FULL, code & 8);
+            auto lanes_of = [&](int k) {
+                return bn & ((k & 1) ? b0 : ~b0) & ((k & 2) ? b1 : ~b1) & ((k & 4) ? b2 : ~b2) & ((k & 8) ? b3 : ~b3);
+            };
+            const int to = near ? code : 0;
+            const int slot = __shfl_sync(FULL, at, to) + __popc(lanes_of(to) & lt);
+            const int limit = __shfl_sync(FULL, lim, to), cell = __shfl_sync(FULL, D, to);
+            at += lane < 9 ? __popc(lanes_of(lane)) : 0;
+            if (near) {
+                if (slot < limit) {
+                    const size_t dst = (size_t)cell * cap + (size_t)slot;
+                    oxy[dst] = xy;
+                    ov[dst] = v;
+                    oz[dst] = vz;
+                } else {
+                    overflow = true;
+                }
+            }
+        }
+        if (__any_sync(FULL, overflow) && lane == 0) atomicOr(d.status, ST_OVERFLOW);
     }
     cp_async_wait_all();
-    if (__any_sync(FULL, overflow) && lane == 0) atomicOr(d.status, ST_OVERFLOW);
 }
 
-// One lane per destination cell (32 cells per warp): the new count is its
-// stayers plus the near movers addressed to it (nine dcount entries, all
-// loads independent); the cells with a far bucket are then finished one at a
-// time by the whole warp (bucket ordered by (source cell, r), then copied).
+// One lane per destination cell (32 cells per warp): the start slots of its
+// near movers, its new count, and its far bucket (ordered by (source cell, r),
+// then copied; by the lane, or by the whole warp where it is long).
 __global__ void __launch_bounds__(SORT_MAXW * 32) k_sort_count(const DevCase *__restrict__ cases,
-                                                         const int *__restrict__ item_start, int ncases, int items) {
+                                                        const int *__restrict__ item_start, int ncases, int items) {
     const int warp = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if (warp * 32 >= items) return;
@@ -588,21 +611,28 @@ __global__ void __launch_bounds__(SORT_MAXW * 32) k_sort_count(const DevCase *__
     if (item < items) {
         ci = find_case(item_start, ncases, item);
         const DevCase &d = cases[ci];
-        const int w = item - item_start[ci];
-        s = w / d.C;
-        c = w - s * d.C;
+        const unsigned w = (unsigned)(item - item_start[ci]);
+        s = (int)d.div_c.quot(w);
+        c = (int)w - s * d.C;
         const DevSpecies &sp = d.sp[s];
-        const int ncy = d.ncy, i = c / ncy, j = c - i * ncy;
+        const int ncy = d.ncy, i = (int)d.div_ncy.quot((unsigned)c), j = c - i * ncy;
         // near movers in: source S = c + (q/3 - 1, q%3 - 1) sends code 8 - q
-        int in = 0;
+        int in[9];
 #pragma unroll
         for (int q = 0; q < 9; q++) {
             const int Si = i + q / 3 - 1, Sj = j + q % 3 - 1;
-            if (Si >= 0 && Si < d.ncx && Sj >= 0 && Sj < ncy) in += sp.dcount[(size_t)(Si * ncy + Sj) * 9 + (8 - q)];
+            in[q] = 0;
+            if (Si >= 0 && Si < d.ncx && Sj >= 0 && Sj < ncy) in[q] = sp.dcount[(size_t)(Si * ncy + Sj) * 9 + (8 - q)];
         }
         limit = sp.cap - sp.nmov[c];
-        out = sp.cnt[c] + in;
+        out = sp.cnt[c];
         nf = d.far_in[(size_t)s * d.C + c];
+#pragma unroll
+        for (int q = 0; q < 9; q++)
+            if (in[q]) {
+                sp.dcount[(size_t)(c + (q / 3 - 1) * ncy + (q % 3 - 1)) * 9 + (8 - q)] = out;
+                out += in[q];
+            }
     }
     bool overflow = false;
     // a bucket of at most FAR_LANE keys is finished by its own lane: keys
@@ -2022,13 +2052,33 @@ cudaError_t launch_sort(const DevCase *cases, const int *item_start, int ncases,
     // at least 8 warps per block: the push gains from them even where Move
     // and Deposit prefer smaller blocks
     const int tpb = 32 * std::min(std::max(lc.warps_per_block, 8), SORT_MAXW);
-    prof::mark(st, "k_sort_push");
-    k_sort_push<<<blocks_for((long long)items * 32, tpb), tpb, (size_t)(tpb / 32) * SORT_PRE * SORT_SLOT * sizeof(float), st>>>(cases, item_start, ncases, items);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
     prof::mark(st, "k_sort_count");
     k_sort_count<<<blocks_for((long long)(items + 31) / 32 * 32, tpb), tpb, 0, st>>>(cases, item_start, ncases, items);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    const int per_warp = balanced_group(items, (long long)sm_count() * 32, SORT_G);
+    prof::mark(st, "k_sort_push");
+    k_sort_push<<<blocks_for(((long long)items + per_warp - 1) / per_warp * 32, tpb), tpb, (size_t)(tpb / 32) * SORT_PRE * SORT_SLOT * sizeof(float), st>>>(cases, item_start, ncases, items, per_warp);
     return cudaGetLastError();
+}
+
+int sm_count() {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 148;
+    return n;
+}
+
+// Cells per warp (at most `most`) for a launch on `warps` resident warps: as
+// many as give every resident warp one group.  With 16 cells per warp
+// whatever their number, a 129x65 case left seven of eight resident
+// warps without work.  (Beyond one wave, fuller batches are worth more than
+// even waves: 13 cells per warp in 2.8 waves ran slower than 16 in 2.3.)
+// Measured on a B200, 16 cells per warp and this: 31 and 15 us at 65x33 with 20
+// particles per cell, 41 and 23 us at 129x65 with 50.
+int balanced_group(long long cells, long long warps, int most) {
+    return (int)std::min<long long>(std::max((cells + warps - 1) / warps, 1LL), most);
 }
 
 cudaError_t launch_mcc_ar(const DevCase *cases, const int *item_start, int ncases, int items, const LaunchCfg &lc,

@@ -17,6 +17,10 @@ struct LaunchCfg {
     int mcc_cells = 16;        // MCC (Ar): consecutive cells per warp, sharing collision batches (1, 2, 4, 8, 16)
 };
 
+// SMs of the current device
+int sm_count();
+// cells per warp of a launch on `warps` resident warps, at most `most`
+int balanced_group(long long cells, long long warps, int most);
 // Move: gather + push + single-cell exit test (src/cuda_Move.cu:181-270)
 cudaError_t launch_move(const DevCase *cases, const int *item_start, int ncases, int items, const LaunchCfg &lc,
                         cudaStream_t st);
