@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "deposit.cuh"
 #include "devutil.cuh"
 #include "hp_math.h"
 #include "hp_rng.h"
@@ -1075,84 +1076,28 @@ __global__ void __launch_bounds__(MCC_TPB, MCC_MINB) k_mcc_ar(const DevCase *__r
 }
 
 // ------------------------------------------------------------------ Deposit
-// DepositAtom (src/cuda_Deposit.cu:289-317): per-cell sums of the four CIC
-// weights; lanes accumulate in FP32, the warp reduces in FP64 and writes one
-// double4 per cell, which the node pass gathers in a fixed order.
-// DEP_G consecutive (species, cell) items per warp: lanes 0..G-1 resolve
-// their item's case, count and array bases together, every lane then loads
-// its first slot of all G cells at once, and the cells are summed one after
-// the other (each lane adds its slots lane, lane + 32, ... of a cell in that
-// order, the warp tree reduces in FP64), so the sums are those of one cell
-// per warp.
-#ifndef DEP_G
-#define DEP_G 2
-#endif
+// DEP_G consecutive (species, cell) items per warp: lanes 0..DEP_G-1 resolve
+// their item's case, count and slots together (deposit.cuh).
 __global__ void __launch_bounds__(512) k_deposit_cells(const DevCase *__restrict__ cases,
                                                        const int *__restrict__ item_start, int ncases, int items) {
-    constexpr int G = DEP_G;
     const int warp = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
-    if (warp * G >= items) return;
+    if ((long long)warp * DEP_G >= items) return;
     int my_n = 0;
     const float2 *my_xy = nullptr;
     double4 *my_cw = nullptr;
-    if (lane < G && warp * G + lane < items) {
-        const int item = warp * G + lane;
+    if (lane < DEP_G && warp * DEP_G + lane < items) {
+        const int item = warp * DEP_G + lane;
         const int ci = find_case(item_start, ncases, item);
         const DevCase &d = cases[ci];
-        const int w = item - item_start[ci];
-        const int s = w / d.C, c = w - s * d.C;
+        const unsigned w = (unsigned)(item - item_start[ci]);
+        const int s = (int)d.div_c.quot(w), c = (int)w - s * d.C;
         const DevSpecies &sp = d.sp[s];
-        const size_t base = (size_t)c * sp.cap;
         my_n = sp.cnt[c];
-        my_xy = sp.xy + base;
+        my_xy = sp.xy + (size_t)c * sp.cap;
         my_cw = d.cw[s] + c;
     }
-    int n[G];
-    const float2 *pxy[G];
-    float2 f0[G];
-#pragma unroll
-    for (int g = 0; g < G; g++) {
-        n[g] = __shfl_sync(FULL, my_n, g);
-        pxy[g] = (const float2 *)__shfl_sync(FULL, (unsigned long long)my_xy, g);
-    }
-    // the first chunk of every cell: slots 0..31 are inside the pool (cap >= 32)
-#pragma unroll
-    for (int g = 0; g < G; g++) {
-        f0[g] = pxy[g] ? pxy[g][lane] : make_float2(0.f, 0.f);
-    }
-#pragma unroll
-    for (int g = 0; g < G; g++) {
-        if (!pxy[g]) continue; // past the last item (warp-uniform)
-        const int ng = n[g];
-        if (ng == 0) { // warp-uniform: the sums of an empty cell are +0, as the tree would give
-            double4 *cw = (double4 *)__shfl_sync(FULL, (unsigned long long)my_cw, g);
-            if (lane == 0) *cw = make_double4(0.0, 0.0, 0.0, 0.0);
-            continue;
-        }
-        float WS = 0.f, WN = 0.f, ES = 0.f, EN = 0.f;
-        auto add = [&](float lx, float ly) {
-            WS += (1 - lx) * (1 - ly);
-            WN += (1 - lx) * ly;
-            ES += lx * (1 - ly);
-            EN += lx * ly;
-        };
-        if (lane < ng) add(f0[g].x, f0[g].y);
-        for (int k0 = 32; k0 < ng; k0 += 128) {
-            float2 f[4];
-#pragma unroll
-            for (int h = 0; h < 4; h++) {
-                const int k = k0 + 32 * h + lane;
-                f[h] = k < ng ? pxy[g][k] : make_float2(0.f, 0.f);
-            }
-#pragma unroll
-            for (int h = 0; h < 4; h++)
-                if (k0 + 32 * h + lane < ng) add(f[h].x, f[h].y);
-        }
-        const double a = warp_sum_d(WS), b = warp_sum_d(WN), e = warp_sum_d(ES), f = warp_sum_d(EN);
-        double4 *cw = (double4 *)__shfl_sync(FULL, (unsigned long long)my_cw, g);
-        if (lane == 0) *cw = make_double4(a, b, e, f);
-    }
+    deposit_group(my_n, my_xy, my_cw);
 }
 
 // The Sort phase's pass over the dielectric crossings Move queued: one block

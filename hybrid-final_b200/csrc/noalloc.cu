@@ -15,6 +15,7 @@
 #include <string>
 
 #include "capi_internal.hpp"
+#include "deposit.cuh"
 
 #define HP_NOALLOC_CELLS (1 << 19) /* species x cells the scratch array holds */
 
@@ -27,33 +28,25 @@ constexpr int kMaxDevices = 64;
 std::mutex g_mu;
 double4 *g_scratch_ptr[kMaxDevices] = {nullptr};
 
-__device__ __forceinline__ double warp_sum_na(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-// per-cell corner sums, as k_deposit_cells: FP32 lane sums, FP64 warp tree
+// per-cell corner sums, as k_deposit_cells: DEP_G cells per warp
 __global__ void __launch_bounds__(256) k_na_cells(const hp::DevCase *__restrict__ dc, double4 *__restrict__ scratch) {
+    using hp::dv::DEP_G;
     const hp::DevCase &d = *dc;
     const int warp = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
-    if (warp >= d.nsp * d.C) return;
-    const int s = warp / d.C, c = warp - s * d.C;
-    const hp::DevSpecies &sp = d.sp[s];
-    const int n = sp.cnt[c];
-    const size_t base = (size_t)c * sp.cap;
-    float WS = 0.f, WN = 0.f, ES = 0.f, EN = 0.f;
-    for (int k = lane; k < n; k += 32) {
-        const float2 f = sp.xy[base + k];
-        const float lx = f.x, ly = f.y;
-        WS += (1 - lx) * (1 - ly);
-        WN += (1 - lx) * ly;
-        ES += lx * (1 - ly);
-        EN += lx * ly;
+    const int lane = threadIdx.x & 31, items = d.nsp * d.C;
+    if (warp * DEP_G >= items) return;
+    int my_n = 0;
+    const float2 *my_xy = nullptr;
+    double4 *my_cw = nullptr;
+    const int item = warp * DEP_G + lane;
+    if (lane < DEP_G && item < items) {
+        const int s = (int)d.div_c.quot((unsigned)item), c = item - s * d.C;
+        const hp::DevSpecies &sp = d.sp[s];
+        my_n = sp.cnt[c];
+        my_xy = sp.xy + (size_t)c * sp.cap;
+        my_cw = scratch + item;
     }
-    const double a = warp_sum_na(WS), b = warp_sum_na(WN), e = warp_sum_na(ES), f = warp_sum_na(EN);
-    if (lane == 0) scratch[warp] = make_double4(a, b, e, f);
+    hp::dv::deposit_group(my_n, my_xy, my_cw);
 }
 
 // node gather and DepositBoundary scaling into the caller's den[nsp*Gsize]
@@ -133,7 +126,7 @@ extern "C" hp_status hp_Deposit_noalloc(hp_case *c, double *den_out, void *strea
         }
         scratch = g_scratch_ptr[c->device];
     }
-    const long long threads = need * 32;
+    const long long threads = (need + hp::dv::DEP_G - 1) / hp::dv::DEP_G * 32;
     k_na_cells<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(c->d_case, scratch);
     e = cudaGetLastError();
     if (e != cudaSuccess) return hpi::cuda_fail(e, "hp_Deposit_noalloc cells");
