@@ -51,52 +51,49 @@ hp_status fast_plan_build(hp_case *const *cases, const std::vector<int> &idx, Fa
     out = FastPlanDev();
     const int n = (int)idx.size();
     if (n == 0) return HP_OK;
-    std::vector<int> items(n + 1, 0);
-    std::vector<GemmProb> st[4];
-    int tiles[4] = {0, 0, 0, 0};
+    FastPlan &p = out.plan;
+    std::vector<int> of_cluster[2], rest, items(1, 0), tiles(1, 0);
     for (int q = 0; q < n; q++) {
         const hp::DevCase &h = cases[q]->h;
-        const int nx = h.fs_nx, ny = h.fs_ny;
-        items[q + 1] = items[q] + nx * ny;
-        const int tn = (nx + FS_TILE - 1) / FS_TILE, tm = (ny + FS_TILE - 1) / FS_TILE;
-        out.plan.final_chunks = std::max(out.plan.final_chunks, (h.G + FS_CHUNK - 1) / FS_CHUNK);
-        GemmProb g[4];
-        std::memset(g, 0, sizeof g);
-        // A1 = X V ; Y = (W^T A1) .* inv ; A2 = Y V^T ; x64 += W A2
-        g[0] = GemmProb{ny, nx, nx, h.fs_x, h.fs_V, h.fs_a1, nullptr, nullptr, 0, 0, 0, 0, tn, 0};
-        g[1] = GemmProb{ny, nx, ny, h.fs_Wt, h.fs_a1, h.fs_y, h.fs_inv, nullptr, 0, 0, 0, 1, tn, 0};
-        g[2] = GemmProb{ny, nx, nx, h.fs_y, h.fs_Vt, h.fs_a1, nullptr, nullptr, 0, 0, 0, 0, tn, 0};
-        g[3] = GemmProb{ny, nx, ny, h.fs_W, h.fs_a1, nullptr, nullptr, h.x64, h.ngy, h.fs_i0, h.fs_j0, 2, tn, 0};
-        for (int k = 0; k < 4; k++) {
-            g[k].tile_start = tiles[k];
-            tiles[k] += tm * tn;
-            st[k].push_back(g[k]);
+        const int nx = h.fs_nx, ny = h.fs_ny, ctas = fs_cluster_ctas(nx, ny);
+        if (ctas) {
+            FastGroup &g = p.groups[ctas == 16];
+            of_cluster[ctas == 16].push_back(idx[q]);
+            g.ctas = ctas;
+            g.smem = std::max(g.smem, fs_cluster_smem(nx, ny));
+            continue;
         }
+        rest.push_back(idx[q]);
+        items.push_back(items.back() + nx * ny);
+        tiles.push_back(tiles.back() + ((nx + FS_TILE - 1) / FS_TILE) * ((ny + FS_TILE - 1) / FS_TILE));
+        p.final_chunks = std::max(p.final_chunks, (h.G + FS_CHUNK - 1) / FS_CHUNK);
     }
-    cudaError_t e;
-    if ((e = cudaMalloc(&out.d_list, sizeof(int) * n)) != cudaSuccess) return cuda_fail(e, "fast plan");
-    if ((e = cudaMalloc(&out.d_items, sizeof(int) * (n + 1))) != cudaSuccess) return cuda_fail(e, "fast plan");
-    if ((e = cudaMalloc(&out.d_probs, sizeof(GemmProb) * 4 * n)) != cudaSuccess) return cuda_fail(e, "fast plan");
-    cudaMemcpy(out.d_list, idx.data(), sizeof(int) * n, cudaMemcpyHostToDevice);
-    cudaMemcpy(out.d_items, items.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice);
-    for (int k = 0; k < 4; k++) {
-        e = cudaMemcpy(out.d_probs + (size_t)k * n, st[k].data(), sizeof(GemmProb) * n, cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) return cuda_fail(e, "fast plan");
-        out.plan.probs[k] = out.d_probs + (size_t)k * n;
-        out.plan.ntiles[k] = tiles[k];
+    std::vector<int> all;
+    size_t at[5];
+    const std::vector<int> *parts[5] = {&of_cluster[0], &of_cluster[1], &rest, &items, &tiles};
+    for (int k = 0; k < 5; k++) {
+        at[k] = all.size();
+        all.insert(all.end(), parts[k]->begin(), parts[k]->end());
     }
-    out.plan.list = out.d_list;
-    out.plan.item_start = out.d_items;
-    out.plan.n = n;
-    out.plan.items = items[n];
-    out.plan.passes = cases[0]->h.fs_passes > 0 ? cases[0]->h.fs_passes : 3;
+    cudaError_t e = cudaMalloc(&out.d_ints, sizeof(int) * all.size());
+    if (e == cudaSuccess) e = cudaMemcpy(out.d_ints, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return cuda_fail(e, "fast plan");
+    for (int k = 0; k < 2; k++) {
+        p.groups[k].list = out.d_ints + at[k];
+        p.groups[k].n = (int)of_cluster[k].size();
+    }
+    p.list = out.d_ints + at[2];
+    p.item_start = out.d_ints + at[3];
+    p.tile_start = out.d_ints + at[4];
+    p.n = (int)rest.size();
+    p.items = items.back();
+    p.tiles = tiles.back();
+    p.passes = cases[0]->h.fs_passes > 0 ? cases[0]->h.fs_passes : 3;
     return HP_OK;
 }
 
 void fast_plan_free(FastPlanDev &f) {
-    cudaFree(f.d_list);
-    cudaFree(f.d_items);
-    cudaFree(f.d_probs);
+    cudaFree(f.d_ints);
     f = FastPlanDev();
 }
 
@@ -502,21 +499,30 @@ hp_status build_device(hp_case *c) {
     if (h.field_mode == 2) {
         // separable inner solve when the operator allows it, else mode 1
         if (build_fast_solver(s, c->fs)) {
-            const size_t nxy = (size_t)c->fs.nx * c->fs.ny;
+            const int nx = c->fs.nx, ny = c->fs.ny;
             h.fs_i0 = c->fs.i0; h.fs_j0 = c->fs.j0; h.fs_nx = c->fs.nx; h.fs_ny = c->fs.ny;
             {
                 const double rtol = c->opts.pcg_rtol > 0 ? c->opts.pcg_rtol : 1e-8;
                 c->fs_passes = c->opts.fs_passes > 0 ? c->opts.fs_passes : (rtol >= 1e-10 ? 2 : 3);
             }
             h.fs_passes = c->fs_passes;
-            TRY(dupload(c, (float **)&h.fs_V, c->fs.V));
-            TRY(dupload(c, (float **)&h.fs_Vt, c->fs.Vt));
-            TRY(dupload(c, (float **)&h.fs_W, c->fs.W));
-            TRY(dupload(c, (float **)&h.fs_Wt, c->fs.Wt));
-            TRY(dupload(c, (float **)&h.fs_inv, c->fs.inv_eig));
-            TRY(dalloc(c, &h.fs_x, nxy));
-            TRY(dalloc(c, &h.fs_a1, nxy));
-            TRY(dalloc(c, &h.fs_y, nxy));
+            h.fs_ldv = (nx + 3) & ~3;
+            h.fs_ldm = (ny + 31) & ~31;
+            auto padded = [](const std::vector<float> &m, int rows, int cols, int ld, bool transpose) {
+                std::vector<float> o((size_t)rows * ld, 0.0f);
+                for (int r = 0; r < rows; r++)
+                    for (int q = 0; q < cols; q++)
+                        o[(size_t)r * ld + q] = transpose ? m[(size_t)q * rows + r] : m[(size_t)r * cols + q];
+                return o;
+            };
+            TRY(dupload(c, (float **)&h.fs_V, padded(c->fs.V, nx, nx, h.fs_ldv, false)));
+            TRY(dupload(c, (float **)&h.fs_Vt, padded(c->fs.Vt, nx, nx, h.fs_ldv, false)));
+            TRY(dupload(c, (float **)&h.fs_W, padded(c->fs.W, ny, ny, h.fs_ldm, false)));
+            TRY(dupload(c, (float **)&h.fs_Wt, padded(c->fs.Wt, ny, ny, h.fs_ldm, false)));
+            TRY(dupload(c, (float **)&h.fs_inv, padded(c->fs.inv_eig, nx, ny, h.fs_ldm, true)));
+            TRY(dalloc(c, &h.fs_xt, (size_t)nx * h.fs_ldm));
+            TRY(dalloc(c, &h.fs_yt, (size_t)nx * h.fs_ldm));
+            if (fs_cluster_ctas(nx, ny) == 0) TRY(dalloc(c, &h.fs_mid, (size_t)ny * h.fs_ldv));
             TRY(dalloc(c, &h.fs_res, 2 + 2 * (size_t)((G + FS_CHUNK - 1) / FS_CHUNK)));
         } else {
             h.field_mode = 1;

@@ -16,8 +16,7 @@ namespace hpi {
 // descriptor array the kernels see).
 struct FastPlanDev {
     hp::FastPlan plan;
-    int *d_list = nullptr, *d_items = nullptr;
-    hp::GemmProb *d_probs = nullptr;
+    int *d_ints = nullptr; // every list of the plan
 };
 } // namespace hpi
 

@@ -185,9 +185,12 @@ struct DevCase {
     int move_mode;                  // 0 one cell crossing per step (reference), 1 cross until inside a cell
     // separable inner solve (field_mode 2): rectangle of unknowns and scratch
     int fs_i0, fs_j0, fs_nx, fs_ny, fs_passes;
-    float *fs_x;                    // [ny*nx] residual of the symmetrised system
-    float *fs_a1, *fs_y;            // [ny*nx] products
-    const float *fs_V, *fs_Vt, *fs_W, *fs_Wt, *fs_inv;
+    int fs_ldm, fs_ldv;             // row lengths: ny rounded up to 32 floats, nx to 4
+    float *fs_xt, *fs_yt;           // [nx][ldm] residual of the symmetrised system and Y, transposed
+    float *fs_mid;                  // [ny][ldv] first product of a pair (null: solved by a cluster)
+    const float *fs_V, *fs_Vt;      // [nx][ldv]
+    const float *fs_W, *fs_Wt;      // [ny][ldm]
+    const float *fs_inv;            // [nx][ldm] inverse eigenvalues, transposed
     double *fs_res;                 // [2]: final ||r||, ||b||
     // fluid species (metastables, radicals): the continuity solve of
     // src/cuda_Fluid.cu:34-167 and the source cycle of

@@ -235,6 +235,14 @@ cudaError_t launch_fluid_sweeps(const DevCase *cases, int ncases, const FluidPla
         const int w = fluid_sweep_warps(L);
         if (w == 0) return cudaErrorInvalidValue;
         const size_t smem = (size_t)w * 16 * (size_t)L;
+        // The sweeps run beside the step's other kernels on a side stream.  An
+        // SM changes its split between L1 and shared memory only when it is
+        // empty, so blocks of a sweep under a small split keep the blocks of
+        // the field's products and of Move, which need most of it as shared
+        // memory, off their SMs (257x129 Ar/O2: a step of 0.689 ms, 0.622 so).
+        const void *kern = dir == 0 ? (const void *)k_fluid_sweep<0> : (const void *)k_fluid_sweep<1>;
+        cudaError_t ec = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        if (ec != cudaSuccess) return ec;
         if (dir == 0) {
             if (smem > 48 * 1024) cudaFuncSetAttribute(k_fluid_sweep<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             prof::mark(st, "k_fluid_sweep_x");

@@ -2135,7 +2135,7 @@ cudaError_t launch_field(const DevCase *cases, const int *node_items, int ncases
         cudaError_t e = cudaLaunchKernelEx(&cfg, k_pcg<false>, cases, pg.list, pg.n);
         if (e != cudaSuccess) return e;
     }
-    if (fast && fast->n > 0) {
+    if (fast) {
         cudaError_t ef = launch_fast_field(cases, *fast, st);
         if (ef != cudaSuccess) return ef;
     }

@@ -14,7 +14,7 @@ struct LaunchCfg {
     int pcg_block = 512;       // PCG: threads per CTA
     int pcg_cluster_max = 16;  // PCG: upper bound on CTAs per case
     int move_unroll = 1;       // Move: chunks of 32 loaded per iteration (1: k_move, one-chunk prefetch)
-    int mcc_cells = 16;        // MCC (Ar): consecutive cells per warp, sharing collision batches (1, 2, 4, 8, 16)
+    int mcc_cells = 16;        // MCC (Ar): most consecutive cells that share collision batches (1, 2, 4, 8, 16)
 };
 
 // SMs of the current device
@@ -58,28 +58,30 @@ struct PcgGroup {
 // launch shape is outside its range
 cudaError_t launch_pcg_chip(const DevCase *cases, const PcgGroup &pg, cudaStream_t st, bool &done);
 // field_mode 2 (fastsolve.cu): refinement passes with the separable inverse
-struct GemmProb {
-    int M, N, K;
-    const float *A, *B;
-    float *C;
-    const float *S;  // epi 1: elementwise scale of the product
-    double *x64;     // epi 2: x64[(i0 + n) * ngy + (j0 + m)] += product
-    int ngy, i0, j0, epi;
-    int tiles_n, tile_start;
+constexpr int FS_CHUNK = 1024;  // nodes per CTA of the final residual pass; a case's fs_res holds
+                                // 2 + 2 * ceil(G / FS_CHUNK) doubles
+constexpr int FS_TILE = 32;     // edge of the output tiles of a launch per product
+constexpr int FS_CLUSTER_MAX = 10000;    // unknowns up to which one cluster solves a case
+constexpr size_t FS_SMEM_MAX = 220 * 1024;
+// shared memory of the cluster solve of nx x ny unknowns, and the CTAs of its
+// cluster (0: solved by one launch per product)
+size_t fs_cluster_smem(int nx, int ny);
+int fs_cluster_ctas(int nx, int ny);
+struct FastGroup {
+    int ctas = 0;              // CTAs per case
+    const int *list = nullptr; // device: case indices
+    int n = 0;
+    size_t smem = 0;
 };
 struct FastPlan {
-    const int *list = nullptr;       // device: case indices
-    const int *item_start = nullptr; // device: prefix of rectangle sizes [n+1]
-    int n = 0, items = 0;
-    const GemmProb *probs[4] = {nullptr, nullptr, nullptr, nullptr}; // device, one list per product
-    int ntiles[4] = {0, 0, 0, 0};
+    FastGroup groups[2];             // cases solved by one cluster each (8 and 16 CTAs)
+    const int *list = nullptr;       // the other cases: device, case indices,
+    const int *item_start = nullptr; // prefix of rectangle sizes [n+1],
+    const int *tile_start = nullptr; // prefix of output tiles [n+1]
+    int n = 0, items = 0, tiles = 0;
     int passes = 3;
-    int final_chunks = 0; // max over the cases of ceil(G / FS_CHUNK)
+    int final_chunks = 0; // max over those cases of ceil(G / FS_CHUNK)
 };
-// nodes per CTA of the final residual pass; a case's fs_res holds
-// 2 + 2 * ceil(G / FS_CHUNK) doubles
-constexpr int FS_CHUNK = 1024;
-constexpr int FS_TILE = 32; // GEMM output tile edge
 cudaError_t launch_fast_field(const DevCase *cases, const FastPlan &fp, cudaStream_t st);
 cudaError_t launch_field(const DevCase *cases, const int *node_items, int ncases, int n_node_items,
                          const PcgGroup *groups, int ngroups, const FastPlan *fast, cudaStream_t st,
