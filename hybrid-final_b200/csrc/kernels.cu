@@ -14,6 +14,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "deposit.cuh"
 #include "devutil.cuh"
@@ -768,6 +769,7 @@ __global__ void __launch_bounds__(SORT_MAXW * 32) k_sort_count(const DevCase *__
 // particle's arithmetic and draws are exactly those of a lane-per-particle
 // loop, and new particles are still appended in particle order.
 constexpr int MCC_TPB = 256;
+constexpr int MCC_G = 16;     // cells of a group, at most
 constexpr int MCC_RING = 256; // >= 128 new entries per pass + 31 pending
 
 // one ion that passed the null-collision test; returns the channel tallied
@@ -891,19 +893,31 @@ __device__ __forceinline__ int mcc_el_collide(const DevCase &d, const DevSpecies
 // The cells one warp works on, with what its lanes need while colliding.
 struct MccCell {
     int c, ne, ni, add; // cell, electrons and ions before the step, births so far
-    float P1, P2, Pion, bvel;
+    unsigned el24, ion24; // a test word x is a hit when x >> 8 is below these
+    float P1, bvel;
 };
 
-#ifndef MCC_MINB
-#define MCC_MINB 3 // 80 registers: three 256-thread blocks per SM
-#endif
+// The null-collision test as a comparison of integers: hp_u01(x) is
+// ((x >> 8) + 1) 2^-24 exactly, so hp_u01(x) < p is (x >> 8) + 1 < 2^24 p and
+// hp_u01(x) <= p is (x >> 8) + 1 <= 2^24 p (2^24 p is exact in float).  Four
+// conversions to float per lane and test block drop out (they run at a
+// quarter of the rate of the rest).
+__device__ __forceinline__ unsigned test_below(float p) {
+    const float t = ceilf(p * 16777216.0f) - 1.0f;
+    return !(t > 0.0f) ? 0u : t >= 16777216.0f ? 16777216u : (unsigned)t;
+}
+__device__ __forceinline__ unsigned test_at_most(float p) {
+    const float t = floorf(p * 16777216.0f);
+    return !(t > 0.0f) ? 0u : t >= 16777216.0f ? 16777216u : (unsigned)t;
+}
+constexpr int MCC_WARPS = 24; // resident warps per SM: 80 registers
+constexpr int MCC_MINB = MCC_WARPS * 32 / MCC_TPB;
 
-// Ions of up to G consecutive cells of one case, then their electrons.  Each
-// queue entry is (slot | cell-in-group << 24, test draw); the queue is
+// Ions of up to MCC_G consecutive cells of one case, then their electrons.  Each
+// queue entry is (slot | cell-in-group << 24, test word); the queue is
 // drained 32 colliders at a time, so the cells of a group share collision
-// batches.  A cell's new pairs are appended behind its own particles in
+// batches.  The test word goes with the entry.  A cell's new pairs are appended behind its own particles in
 // queue order, which is the cell's particle order.
-template <int G>
 __device__ __forceinline__ void mcc_ar_cells(const DevCase &d, int c0, int n, int2 *ring, MccCell *cs,
                                              unsigned *tally, int lane, unsigned lt, bool &overflow) {
     const uint32_t step = (uint32_t)(*d.tstep);
@@ -918,21 +932,22 @@ __device__ __forceinline__ void mcc_ar_cells(const DevCase &d, int c0, int n, in
         m.ni = ion.cnt[c];
         m.add = 0;
         m.P1 = d.prob[c];
-        m.P2 = d.prob[d.C + c];
-        m.Pion = d.prob[2 * d.C + c];
+        m.el24 = test_below(d.prob[d.C + c]);
+        m.ion24 = test_at_most(d.prob[2 * d.C + c]);
         m.bvel = d.back_vel1[i * d.ngy + j];
         cs[lane] = m;
     }
-    for (int k = lane; k < G * 8; k += 32) tally[k] = 0u;
+    for (int k = lane; k < n * 8; k += 32) tally[k] = 0u;
     __syncwarp();
     int head = 0, tail = 0;
-    // queue the slots of `hits` (four per lane, slot k + t) behind the tail
-    auto enqueue = [&](unsigned hits, int k, int cl, const float *R) {
+    // queue the slots of `hits` (four per lane, slot k + t, with their test words) behind the tail
+    auto enqueue = [&](unsigned hits, int k, int cl, hp_u4 u) {
         int total;
         int pos = tail + lower_lane_hits(hits, lt, total);
 #pragma unroll
         for (int t = 0; t < 4; t++)
-            if ((hits >> t) & 1u) ring[(pos++) & (MCC_RING - 1)] = make_int2((k + t) | (cl << 24), __float_as_int(R[t]));
+            if ((hits >> t) & 1u)
+                ring[(pos++) & (MCC_RING - 1)] = make_int2((k + t) | (cl << 24), (int)hp_word(u, (uint32_t)t));
         tail += total;
         __syncwarp();
     };
@@ -953,18 +968,18 @@ __device__ __forceinline__ void mcc_ar_cells(const DevCase &d, int c0, int n, in
     };
     for (int cl = 0; cl < n; cl++) {
         const int c = cs[cl].c, ni = cs[cl].ni;
-        const float Pion = cs[cl].Pion;
+        const unsigned below = cs[cl].ion24;
         for (int k0 = 0; k0 < ni; k0 += 128) {
             const int k = k0 + 4 * lane;
             unsigned hits = 0;
-            float R[4] = {0.f, 0.f, 0.f, 0.f};
+            hp_u4 u = {0u, 0u, 0u, 0u};
             if (k < ni) {
-                const hp_u4 u = hp_test_block(d.seed, (uint32_t)(k >> 2), (uint32_t)c, step, 1u, 0u);
+                u = hp_test_block(d.seed, (uint32_t)(k >> 2), (uint32_t)c, step, 1u, 0u);
 #pragma unroll
                 for (int t = 0; t < 4; t++)
-                    if (k + t < ni && hp_u01(hp_word(u, (uint32_t)t)) <= Pion) hits |= 1u << t;
+                    if (k + t < ni && (hp_word(u, (uint32_t)t) >> 8) < below) hits |= 1u << t;
             }
-            enqueue(hits, k, cl, R);
+            enqueue(hits, k, cl, u);
             while (tail - head >= 32) ion_batch();
         }
     }
@@ -981,7 +996,8 @@ __device__ __forceinline__ void mcc_ar_cells(const DevCase &d, int c0, int n, in
             const int c = cs[q].c;
             hp_stream rs;
             hp_stream_init(&rs, d.seed, (uint32_t)k, (uint32_t)c, step, 0u);
-            ch = mcc_el_collide(d, el, (size_t)c * el.cap + k, rs, __int_as_float(ent.y), cs[q].P1, cs[q].bvel, np);
+            ch = mcc_el_collide(d, el, (size_t)c * el.cap + k, rs, hp_u01((uint32_t)ent.y), cs[q].P1, cs[q].bvel,
+                                np);
             if (ch >= 0) atomicAdd(&tally[q * 8 + ch], 1u);
         }
         const bool create = ch >= 3;
@@ -1012,26 +1028,23 @@ __device__ __forceinline__ void mcc_ar_cells(const DevCase &d, int c0, int n, in
     };
     for (int cl = 0; cl < n; cl++) {
         const int c = cs[cl].c, ne = cs[cl].ne;
-        const float P2 = cs[cl].P2;
+        const unsigned below = cs[cl].el24;
         for (int k0 = 0; k0 < ne; k0 += 128) {
             const int k = k0 + 4 * lane;
             unsigned hits = 0;
-            float R[4] = {0.f, 0.f, 0.f, 0.f};
+            hp_u4 w = {0u, 0u, 0u, 0u}; // the words that hit
             if (k < ne) {
                 const unsigned live = k + 4 <= ne ? 0xFu : (1u << (ne - k)) - 1u;
                 for (int jj = 0; jj < d.mcc_n && (hits != live); jj++) {
                     const hp_u4 u = hp_test_block(d.seed, (uint32_t)(k >> 2), (uint32_t)c, step, 0u, (uint32_t)jj);
-#pragma unroll
-                    for (int t = 0; t < 4; t++) {
-                        const float r = hp_u01(hp_word(u, (uint32_t)t));
-                        if (((live & ~hits) >> t) & 1u && r < P2) {
-                            hits |= 1u << t;
-                            R[t] = r;
-                        }
-                    }
+                    const unsigned open = live & ~hits;
+                    if ((open & 1u) && (u.x >> 8) < below) { hits |= 1u; w.x = u.x; }
+                    if ((open & 2u) && (u.y >> 8) < below) { hits |= 2u; w.y = u.y; }
+                    if ((open & 4u) && (u.z >> 8) < below) { hits |= 4u; w.z = u.z; }
+                    if ((open & 8u) && (u.w >> 8) < below) { hits |= 8u; w.w = u.w; }
                 }
             }
-            enqueue(hits, k, cl, R);
+            enqueue(hits, k, cl, w);
             while (tail - head >= 32) el_batch();
         }
     }
@@ -1050,26 +1063,23 @@ __device__ __forceinline__ void mcc_ar_cells(const DevCase &d, int c0, int n, in
     __syncwarp();
 }
 
-template <int G>
+// One warp per group of `group` <= MCC_G consecutive cells.
 __global__ void __launch_bounds__(MCC_TPB, MCC_MINB) k_mcc_ar(const DevCase *__restrict__ cases,
                                                               const int *__restrict__ item_start, int ncases,
-                                                              int items) {
+                                                              int items, int group) {
     __shared__ int2 ring_s[MCC_TPB / 32][MCC_RING];
-    __shared__ MccCell cell_s[MCC_TPB / 32][G];
-    __shared__ unsigned tally_s[MCC_TPB / 32][G * 8];
+    __shared__ MccCell cell_s[MCC_TPB / 32][MCC_G];
+    __shared__ unsigned tally_s[MCC_TPB / 32][MCC_G * 8];
     const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int first = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5) * G;
-    if (first >= items) return;
     const unsigned lt = lanemask_lt();
-    const int end = min(first + G, items);
-    bool overflow = false;
+    const int first = ((int)blockIdx.x * (MCC_TPB / 32) + wl) * group, end = min(first + group, items);
     // a group that straddles two cases of a batch runs as two groups
     for (int g0 = first; g0 < end;) {
         const int ci = find_case(item_start, ncases, g0);
         const int g1 = min(end, item_start[ci + 1]);
         const DevCase &d = cases[ci];
-        overflow = false;
-        mcc_ar_cells<G>(d, g0 - item_start[ci], g1 - g0, ring_s[wl], cell_s[wl], tally_s[wl], lane, lt, overflow);
+        bool overflow = false;
+        mcc_ar_cells(d, g0 - item_start[ci], g1 - g0, ring_s[wl], cell_s[wl], tally_s[wl], lane, lt, overflow);
         if (__any_sync(FULL, overflow) && lane == 0) atomicOr(d.status, ST_OVERFLOW);
         g0 = g1;
     }
@@ -1874,7 +1884,15 @@ __global__ void __launch_bounds__(PW_T) k_circuit(DevCase *cases, int ncases) {
         surf[i] = (float)d.pw->surf[i];
         pois[i] = (float)part[0][i];
     }
-    hp_circuit_step(nc, d.cc_a, d.lap_sig, vt, C.qconv, surf, pois, C.q, C.phi, C.pois, d.circuit_mode);
+    // one thread's latency: with the number of conductors a constant the small
+    // matrices stay in registers
+    auto solve = [&](auto n) {
+        hp_circuit_step(decltype(n)::value, d.cc_a, d.lap_sig, vt, C.qconv, surf, pois, C.q, C.phi, C.pois,
+                        d.circuit_mode);
+    };
+    if (nc == 2) solve(std::integral_constant<int, 2>());
+    else if (nc == 3) solve(std::integral_constant<int, 3>());
+    else hp_circuit_step(nc, d.cc_a, d.lap_sig, vt, C.qconv, surf, pois, C.q, C.phi, C.pois, d.circuit_mode);
     (void)ncases;
 }
 
@@ -2029,14 +2047,9 @@ int balanced_group(long long cells, long long warps, int most) {
 cudaError_t launch_mcc_ar(const DevCase *cases, const int *item_start, int ncases, int items, const LaunchCfg &lc,
                           cudaStream_t st) {
     if (items <= 0) return cudaSuccess;
-    const int g = lc.mcc_cells;
-    const long long threads = (long long)((items + g - 1) / g) * 32;
+    const int group = balanced_group(items, (long long)sm_count() * MCC_WARPS, lc.mcc_cells);
     prof::mark(st, "k_mcc_ar");
-    if (g == 1) k_mcc_ar<1><<<blocks_for(threads, MCC_TPB), MCC_TPB, 0, st>>>(cases, item_start, ncases, items);
-    else if (g == 2) k_mcc_ar<2><<<blocks_for(threads, MCC_TPB), MCC_TPB, 0, st>>>(cases, item_start, ncases, items);
-    else if (g == 8) k_mcc_ar<8><<<blocks_for(threads, MCC_TPB), MCC_TPB, 0, st>>>(cases, item_start, ncases, items);
-    else if (g == 16) k_mcc_ar<16><<<blocks_for(threads, MCC_TPB), MCC_TPB, 0, st>>>(cases, item_start, ncases, items);
-    else k_mcc_ar<4><<<blocks_for(threads, MCC_TPB), MCC_TPB, 0, st>>>(cases, item_start, ncases, items);
+    k_mcc_ar<<<blocks_for(((long long)items + group - 1) / group * 32, MCC_TPB), MCC_TPB, 0, st>>>(cases, item_start, ncases, items, group);
     return cudaGetLastError();
 }
 

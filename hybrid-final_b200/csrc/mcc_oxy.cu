@@ -482,9 +482,8 @@ __device__ void ion_collide(const DevCase &d, int s, float vx, float vy, float v
 
 __device__ __forceinline__ bool is_hole(float x) { return x != x; }
 
-#ifndef OXY_MINB
-#define OXY_MINB 5 // 96 registers: five 128-thread blocks per SM
-#endif
+constexpr int OXY_WARPS = 20; // resident warps per SM: 96 registers
+constexpr int OXY_MINB = OXY_WARPS * 32 / OXY_TPB;
 #ifndef OXY_G
 #define OXY_G 4
 #endif
@@ -747,18 +746,18 @@ __device__ __forceinline__ void mcc_oxy_cells(const DevCase &d, int c0, int ncel
     }
 }
 
+// one warp per group of `group` <= G consecutive cells
 template <int GAS, int G>
 __global__ void __launch_bounds__(OXY_TPB, OXY_MINB) k_mcc_oxy(const DevCase *__restrict__ cases,
-                                                     const int *__restrict__ item_start, int ncases, int items) {
+                                                     const int *__restrict__ item_start, int ncases, int items,
+                                                     int group) {
     __shared__ int ring_s[OXY_TPB / 32][OXY_RING];
     __shared__ int holes_s[OXY_TPB / 32][G][NSP_ARO2][HOLE_CAP];
     __shared__ CellProb prob_s[OXY_TPB / 32][G];
     __shared__ OxyCell cell_s[OXY_TPB / 32][G];
     const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int first = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5) * G;
-    if (first >= items) return;
     const unsigned lt = lanemask_lt();
-    const int end = min(first + G, items);
+    const int first = ((int)blockIdx.x * (OXY_TPB / 32) + wl) * group, end = min(first + group, items);
     // a group that straddles two cases of a batch runs as two groups
     for (int g0 = first; g0 < end;) {
         const int ci = find_case(item_start, ncases, g0);
@@ -778,10 +777,11 @@ cudaError_t launch_mcc_oxy(const DevCase *cases, const int *item_start, int ncas
                            cudaStream_t st) {
     if (items <= 0) return cudaSuccess;
     constexpr int G = OXY_G;
-    const unsigned nb = (unsigned)(((items + G - 1) / G * 32LL + OXY_TPB - 1) / OXY_TPB);
+    const int group = balanced_group(items, (long long)sm_count() * OXY_WARPS, G);
+    const unsigned nb = (unsigned)((((long long)items + group - 1) / group * 32 + OXY_TPB - 1) / OXY_TPB);
     prof::mark(st, "k_mcc_oxy");
-    if (gas == 2) k_mcc_oxy<2, G><<<nb, OXY_TPB, 0, st>>>(cases, item_start, ncases, items);
-    else if (gas == 1) k_mcc_oxy<1, G><<<nb, OXY_TPB, 0, st>>>(cases, item_start, ncases, items);
+    if (gas == 2) k_mcc_oxy<2, G><<<nb, OXY_TPB, 0, st>>>(cases, item_start, ncases, items, group);
+    else if (gas == 1) k_mcc_oxy<1, G><<<nb, OXY_TPB, 0, st>>>(cases, item_start, ncases, items, group);
     else return cudaErrorNotSupported;
     return cudaGetLastError();
 }
