@@ -25,6 +25,17 @@ __device__ __forceinline__ int find_case(const int *start, int n, int w) {
     return lo;
 }
 
+// First statement of every kernel of a step: wait until the kernel before it
+// in the stream has finished and its writes are visible (nothing is read
+// before), then let the next one be put on the SMs that have room, where it
+// waits in the same place.  With a launch by launch_next (kernels.cuh) the
+// next kernel's launch latency then passes while this one runs; without it
+// both instructions do nothing.
+__device__ __forceinline__ void enter_kernel() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ unsigned lanemask_lt() {
     unsigned m;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));

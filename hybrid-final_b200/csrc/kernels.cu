@@ -268,6 +268,7 @@ constexpr int MOVE_SLOT = 5 * 32; // floats per ring slot: (x, y), (vx, vy), vz
 template <int R>
 __global__ void __launch_bounds__(512, MOVE_MINB) k_move(const DevCase *__restrict__ cases,
                                                  const int *__restrict__ item_start, int ncases, int items) {
+    enter_kernel();
     extern __shared__ __align__(16) float move_ring_s[];
     float *const ring = move_ring_s + (threadIdx.x >> 5) * (R * MOVE_SLOT);
     const int warp = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
@@ -473,6 +474,7 @@ constexpr int SORT_SLOT = 5 * 32 + 8; // floats per ring slot: (x, y), (vx, vy),
 __global__ void __launch_bounds__(SORT_MAXW * 32, SORT_MINB) k_sort_push(const DevCase *__restrict__ cases,
                                                            const int *__restrict__ item_start, int ncases, int items,
                                                            int per_warp) {
+    enter_kernel();
     extern __shared__ __align__(16) float sort_ring_s[];
     const int warp = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
@@ -605,6 +607,7 @@ __global__ void __launch_bounds__(SORT_MAXW * 32, SORT_MINB) k_sort_push(const D
 // then copied; by the lane, or by the whole warp where it is long).
 __global__ void __launch_bounds__(SORT_MAXW * 32) k_sort_count(const DevCase *__restrict__ cases,
                                                         const int *__restrict__ item_start, int ncases, int items) {
+    enter_kernel();
     const int warp = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if (warp * 32 >= items) return;
@@ -1067,6 +1070,7 @@ __device__ __forceinline__ void mcc_ar_cells(const DevCase &d, int c0, int n, in
 __global__ void __launch_bounds__(MCC_TPB, MCC_MINB) k_mcc_ar(const DevCase *__restrict__ cases,
                                                               const int *__restrict__ item_start, int ncases,
                                                               int items, int group) {
+    enter_kernel();
     __shared__ int2 ring_s[MCC_TPB / 32][MCC_RING];
     __shared__ MccCell cell_s[MCC_TPB / 32][MCC_G];
     __shared__ unsigned tally_s[MCC_TPB / 32][MCC_G * 8];
@@ -1090,6 +1094,7 @@ __global__ void __launch_bounds__(MCC_TPB, MCC_MINB) k_mcc_ar(const DevCase *__r
 // their item's case, count and slots together (deposit.cuh).
 __global__ void __launch_bounds__(512) k_deposit_cells(const DevCase *__restrict__ cases,
                                                        const int *__restrict__ item_start, int ncases, int items) {
+    enter_kernel();
     const int warp = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if ((long long)warp * DEP_G >= items) return;
@@ -1114,6 +1119,7 @@ __global__ void __launch_bounds__(512) k_deposit_cells(const DevCase *__restrict
 // per case, then the queue is emptied for the next step.  The fixed-point
 // sums make the result independent of the order of the entries.
 __global__ void __launch_bounds__(256) k_surface(const DevCase *__restrict__ cases, int ncases) {
+    enter_kernel();
     const DevCase &d = cases[blockIdx.x];
     if (!d.sig) return;
     const int n = min(*d.dq_n, d.dq_cap);
@@ -1149,6 +1155,7 @@ __device__ __forceinline__ double surface_charge(const DevCase &d, int n) {
 // DepositBoundary + SumSource + PCG_Set (src/cuda_Deposit.cu:277-288,35-104,30-34)
 __global__ void __launch_bounds__(256) k_deposit_nodes(const DevCase *__restrict__ cases,
                                                        const int *__restrict__ item_start, int ncases, int items) {
+    enter_kernel();
     const int t = (int)(blockIdx.x * (unsigned)blockDim.x + threadIdx.x);
     if (t >= items) return;
     const int ci = find_case(item_start, ncases, t);
@@ -1198,6 +1205,7 @@ __device__ __forceinline__ double smooth_121(const int *dr, const double *v, int
 
 __global__ void __launch_bounds__(256) k_smooth(const DevCase *__restrict__ cases, const int *__restrict__ item_start,
                                                 int ncases, int items, int pass, int along_y) {
+    enter_kernel();
     const int t = (int)(blockIdx.x * (unsigned)blockDim.x + threadIdx.x);
     if (t >= items) return;
     const int ci = find_case(item_start, ncases, t);
@@ -1215,6 +1223,7 @@ __global__ void __launch_bounds__(256) k_smooth(const DevCase *__restrict__ case
 // SumSource + PCG_Set after the smoothing: rho/eps0 and the right-hand side
 __global__ void __launch_bounds__(256) k_source(const DevCase *__restrict__ cases, const int *__restrict__ item_start,
                                                 int ncases, int items) {
+    enter_kernel();
     const int t = (int)(blockIdx.x * (unsigned)blockDim.x + threadIdx.x);
     if (t >= items) return;
     const int ci = find_case(item_start, ncases, t);
@@ -1587,6 +1596,7 @@ __device__ __forceinline__ float cond_voltage(const DevCase &d, int k, double ti
 // order and precision (float accumulation, V_k(t) from a double sine).
 __global__ void __launch_bounds__(256) k_potential(const DevCase *__restrict__ cases, const int *__restrict__ item_start,
                                                    int ncases, int items) {
+    enter_kernel();
     const int t = (int)(blockIdx.x * (unsigned)blockDim.x + threadIdx.x);
     if (t >= items) return;
     const int ci = find_case(item_start, ncases, t);
@@ -1649,6 +1659,7 @@ __device__ float cond_sigma_at(const DevCase &d, int n) {
 // reference's face, corner and boundary special cases.
 __global__ void __launch_bounds__(256) k_efield(const DevCase *__restrict__ cases, const int *__restrict__ item_start,
                                                 int ncases, int items) {
+    enter_kernel();
     const int t = (int)(blockIdx.x * (unsigned)blockDim.x + threadIdx.x);
     if (t >= items) return;
     const int ci = find_case(item_start, ncases, t);
@@ -1783,6 +1794,7 @@ __global__ void __launch_bounds__(256) k_efield(const DevCase *__restrict__ case
 // controller.  hp_powf stands for the reference's double pow.
 constexpr int PW_T = 256;
 __global__ void __launch_bounds__(PW_T) k_power(DevCase *cases, int ncases) {
+    enter_kernel();
     const DevCase &d = cases[blockIdx.x];
     if (!d.pw) return;
     __shared__ double part[PW_T][DMAXCOND];
@@ -1851,6 +1863,7 @@ __global__ void __launch_bounds__(PW_T) k_power(DevCase *cases, int ncases) {
 // last step's surface charge and absorbed charge.  k_potential then puts the
 // conductors at the circuit's potentials.
 __global__ void __launch_bounds__(PW_T) k_circuit(DevCase *cases, int ncases) {
+    enter_kernel();
     const DevCase &d = cases[blockIdx.x];
     if (!d.cs) return;
     __shared__ double part[PW_T][HP_CIRCUIT_MAX];
@@ -1897,12 +1910,14 @@ __global__ void __launch_bounds__(PW_T) k_circuit(DevCase *cases, int ncases) {
 }
 
 __global__ void k_advance(const DevCase *__restrict__ cases, int ncases) {
+    enter_kernel();
     const int t = (int)(blockIdx.x * (unsigned)blockDim.x + threadIdx.x);
     if (t < ncases) *cases[t].tstep += 1;
 }
 
 __global__ void __launch_bounds__(256) k_accumulate(const DevCase *__restrict__ cases,
                                                     const int *__restrict__ item_start, int ncases, int items) {
+    enter_kernel();
     const int t = (int)(blockIdx.x * (unsigned)blockDim.x + threadIdx.x);
     if (t >= items) return;
     const int ci = find_case(item_start, ncases, t);
@@ -1924,6 +1939,7 @@ __global__ void __launch_bounds__(256) k_accumulate(const DevCase *__restrict__ 
 // 64-bit histogram: integer counts, so the result does not depend on order.
 __global__ void __launch_bounds__(256) k_eedf(const DevCase *__restrict__ cases, const int *__restrict__ item_start,
                                               int ncases, int items) {
+    enter_kernel();
     __shared__ unsigned int h[HP_EEDF_BINS + 1];
     __shared__ int case_of_block;
     for (int b = threadIdx.x; b <= HP_EEDF_BINS; b += blockDim.x) h[b] = 0;
@@ -1990,16 +2006,16 @@ cudaError_t launch_move(const DevCase *cases, const int *item_start, int ncases,
     const unsigned nb = blocks_for((long long)items * 32, tpb);
     prof::mark(st, "k_move");
     const size_t slot = (size_t)(tpb / 32) * MOVE_SLOT * sizeof(float);
-    if (lc.move_unroll == 2) k_move<MOVE_RING - 1><<<nb, tpb, (MOVE_RING - 1) * slot, st>>>(cases, item_start, ncases, items);
-    else if (lc.move_unroll == 4) k_move<MOVE_RING + 2><<<nb, tpb, (MOVE_RING + 2) * slot, st>>>(cases, item_start, ncases, items);
-    else k_move<MOVE_RING><<<nb, tpb, MOVE_RING * slot, st>>>(cases, item_start, ncases, items);
+    if (lc.move_unroll == 2) launch_next(k_move<MOVE_RING - 1>, nb, tpb, (MOVE_RING - 1) * slot, st, cases, item_start, ncases, items);
+    else if (lc.move_unroll == 4) launch_next(k_move<MOVE_RING + 2>, nb, tpb, (MOVE_RING + 2) * slot, st, cases, item_start, ncases, items);
+    else launch_next(k_move<MOVE_RING>, nb, tpb, MOVE_RING * slot, st, cases, item_start, ncases, items);
     return cudaGetLastError();
 }
 
 cudaError_t launch_power(DevCase *cases, int ncases, cudaStream_t st) {
     if (ncases <= 0) return cudaSuccess;
     prof::mark(st, "k_power");
-    k_power<<<ncases, PW_T, 0, st>>>(cases, ncases);
+    launch_next(k_power, ncases, PW_T, 0, st, cases, ncases);
     return cudaGetLastError();
 }
 
@@ -2008,7 +2024,7 @@ cudaError_t launch_sort(const DevCase *cases, const int *item_start, int ncases,
     if (items <= 0) return cudaSuccess;
     if (surface) {
         prof::mark(st, "k_surface");
-        k_surface<<<ncases, 256, 0, st>>>(cases, ncases);
+        launch_next(k_surface, ncases, 256, 0, st, cases, ncases);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
@@ -2016,12 +2032,13 @@ cudaError_t launch_sort(const DevCase *cases, const int *item_start, int ncases,
     // and Deposit prefer smaller blocks
     const int tpb = 32 * std::min(std::max(lc.warps_per_block, 8), SORT_MAXW);
     prof::mark(st, "k_sort_count");
-    k_sort_count<<<blocks_for((long long)(items + 31) / 32 * 32, tpb), tpb, 0, st>>>(cases, item_start, ncases, items);
+    launch_next(k_sort_count, blocks_for((long long)(items + 31) / 32 * 32, tpb), tpb, 0, st, cases, item_start, ncases, items);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const int per_warp = balanced_group(items, (long long)sm_count() * 32, SORT_G);
     prof::mark(st, "k_sort_push");
-    k_sort_push<<<blocks_for(((long long)items + per_warp - 1) / per_warp * 32, tpb), tpb, (size_t)(tpb / 32) * SORT_PRE * SORT_SLOT * sizeof(float), st>>>(cases, item_start, ncases, items, per_warp);
+    launch_next(k_sort_push, blocks_for(((long long)items + per_warp - 1) / per_warp * 32, tpb), tpb,
+                (size_t)(tpb / 32) * SORT_PRE * SORT_SLOT * sizeof(float), st, cases, item_start, ncases, items, per_warp);
     return cudaGetLastError();
 }
 
@@ -2049,8 +2066,8 @@ cudaError_t launch_mcc_ar(const DevCase *cases, const int *item_start, int ncase
     if (items <= 0) return cudaSuccess;
     const int group = balanced_group(items, (long long)sm_count() * MCC_WARPS, lc.mcc_cells);
     prof::mark(st, "k_mcc_ar");
-    k_mcc_ar<<<blocks_for(((long long)items + group - 1) / group * 32, MCC_TPB), MCC_TPB, 0, st>>>(cases, item_start, ncases, items, group);
-    return cudaGetLastError();
+    return launch_next(k_mcc_ar, blocks_for(((long long)items + group - 1) / group * 32, MCC_TPB), MCC_TPB, 0, st, cases,
+                       item_start, ncases, items, group);
 }
 
 cudaError_t launch_deposit(const DevCase *cases, const int *cell_items, const int *node_items, int ncases,
@@ -2058,22 +2075,22 @@ cudaError_t launch_deposit(const DevCase *cases, const int *cell_items, const in
     const int tpb = 32 * std::min(std::max(lc.warps_per_block, 1), 16);
     if (n_cell_items > 0) {
         prof::mark(st, "k_deposit_cells");
-        k_deposit_cells<<<blocks_for((long long)(n_cell_items + DEP_G - 1) / DEP_G * 32, tpb), tpb, 0, st>>>(cases, cell_items, ncases, n_cell_items);
+        launch_next(k_deposit_cells, blocks_for((long long)(n_cell_items + DEP_G - 1) / DEP_G * 32, tpb), tpb, 0, st, cases, cell_items, ncases, n_cell_items);
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (n_node_items > 0) {
         prof::mark(st, "k_deposit_nodes");
-        k_deposit_nodes<<<blocks_for(n_node_items, 256), 256, 0, st>>>(cases, node_items, ncases, n_node_items);
+        launch_next(k_deposit_nodes, blocks_for(n_node_items, 256), 256, 0, st, cases, node_items, ncases, n_node_items);
     }
     if (max_smt > 0 && n_node_items > 0) {
         for (int p = 0; p < max_smt; p++)
             for (int yy = 0; yy < 2; yy++) {
                 prof::mark(st, "k_smooth");
-                k_smooth<<<blocks_for(n_node_items, 256), 256, 0, st>>>(cases, node_items, ncases, n_node_items, p, yy);
+                launch_next(k_smooth, blocks_for(n_node_items, 256), 256, 0, st, cases, node_items, ncases, n_node_items, p, yy);
             }
         prof::mark(st, "k_source");
-        k_source<<<blocks_for(n_node_items, 256), 256, 0, st>>>(cases, node_items, ncases, n_node_items);
+        launch_next(k_source, blocks_for(n_node_items, 256), 256, 0, st, cases, node_items, ncases, n_node_items);
     }
     return cudaGetLastError();
 }
@@ -2154,16 +2171,16 @@ cudaError_t launch_field(const DevCase *cases, const int *node_items, int ncases
     }
     if (circuit) {
         prof::mark(st, "k_circuit");
-        k_circuit<<<ncases, PW_T, 0, st>>>(const_cast<DevCase *>(cases), ncases);
+        launch_next(k_circuit, ncases, PW_T, 0, st, const_cast<DevCase *>(cases), ncases);
         cudaError_t ec = cudaGetLastError();
         if (ec != cudaSuccess) return ec;
     }
     prof::mark(st, "k_potential");
-    k_potential<<<blocks_for(n_node_items, 256), 256, 0, st>>>(cases, node_items, ncases, n_node_items);
+    launch_next(k_potential, blocks_for(n_node_items, 256), 256, 0, st, cases, node_items, ncases, n_node_items);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     prof::mark(st, "k_efield");
-    k_efield<<<blocks_for(n_node_items, 256), 256, 0, st>>>(cases, node_items, ncases, n_node_items);
+    launch_next(k_efield, blocks_for(n_node_items, 256), 256, 0, st, cases, node_items, ncases, n_node_items);
     return cudaGetLastError();
 }
 
@@ -2174,14 +2191,14 @@ cudaError_t launch_scatter(const DevSpecies &sp, int C, const int *start, const 
 
 cudaError_t launch_advance(const DevCase *cases, int ncases, cudaStream_t st) {
     prof::mark(st, "k_advance");
-    k_advance<<<blocks_for(ncases, 128), 128, 0, st>>>(cases, ncases);
+    launch_next(k_advance, blocks_for(ncases, 128), 128, 0, st, cases, ncases);
     return cudaGetLastError();
 }
 
 cudaError_t launch_eedf(const DevCase *cases, const int *cell_items, int ncases, int n_cell_items, cudaStream_t st) {
     if (n_cell_items <= 0) return cudaSuccess;
     prof::mark(st, "k_eedf");
-    k_eedf<<<blocks_for((long long)n_cell_items * 32, 256), 256, 0, st>>>(cases, cell_items, ncases, n_cell_items);
+    launch_next(k_eedf, blocks_for((long long)n_cell_items * 32, 256), 256, 0, st, cases, cell_items, ncases, n_cell_items);
     return cudaGetLastError();
 }
 
@@ -2189,7 +2206,7 @@ cudaError_t launch_accumulate(const DevCase *cases, const int *node_items, int n
                               cudaStream_t st) {
     if (n_node_items <= 0) return cudaSuccess;
     prof::mark(st, "k_accumulate");
-    k_accumulate<<<blocks_for(n_node_items, 256), 256, 0, st>>>(cases, node_items, ncases, n_node_items);
+    launch_next(k_accumulate, blocks_for(n_node_items, 256), 256, 0, st, cases, node_items, ncases, n_node_items);
     return cudaGetLastError();
 }
 

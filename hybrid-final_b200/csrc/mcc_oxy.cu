@@ -751,6 +751,7 @@ template <int GAS, int G>
 __global__ void __launch_bounds__(OXY_TPB, OXY_MINB) k_mcc_oxy(const DevCase *__restrict__ cases,
                                                      const int *__restrict__ item_start, int ncases, int items,
                                                      int group) {
+    enter_kernel();
     __shared__ int ring_s[OXY_TPB / 32][OXY_RING];
     __shared__ int holes_s[OXY_TPB / 32][G][NSP_ARO2][HOLE_CAP];
     __shared__ CellProb prob_s[OXY_TPB / 32][G];
@@ -780,8 +781,8 @@ cudaError_t launch_mcc_oxy(const DevCase *cases, const int *item_start, int ncas
     const int group = balanced_group(items, (long long)sm_count() * OXY_WARPS, G);
     const unsigned nb = (unsigned)((((long long)items + group - 1) / group * 32 + OXY_TPB - 1) / OXY_TPB);
     prof::mark(st, "k_mcc_oxy");
-    if (gas == 2) k_mcc_oxy<2, G><<<nb, OXY_TPB, 0, st>>>(cases, item_start, ncases, items, group);
-    else if (gas == 1) k_mcc_oxy<1, G><<<nb, OXY_TPB, 0, st>>>(cases, item_start, ncases, items, group);
+    if (gas == 2) launch_next(k_mcc_oxy<2, G>, nb, OXY_TPB, 0, st, cases, item_start, ncases, items, group);
+    else if (gas == 1) launch_next(k_mcc_oxy<1, G>, nb, OXY_TPB, 0, st, cases, item_start, ncases, items, group);
     else return cudaErrorNotSupported;
     return cudaGetLastError();
 }

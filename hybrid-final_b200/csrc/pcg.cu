@@ -110,6 +110,7 @@ template <> struct Shared<true> { // the whole GPU's
 template <bool GRID, int K>
 __global__ void __launch_bounds__(512, 1) k_pcg_chip(const DevCase *__restrict__ cases, const int *__restrict__ list,
                                                   int nlist, int max_per, int max_ngy) {
+    enter_kernel();
     extern __shared__ float dyn[];
     __shared__ Shared<GRID> sh;
     cg::cluster_group cl = cg::this_cluster();
@@ -494,7 +495,7 @@ cudaError_t launch_pcg_chip(const DevCase *cases, const PcgGroup &pg, cudaStream
         cfg.blockDim = dim3((unsigned)pg.block, 1, 1);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = st;
-        cudaLaunchAttribute attr[1];
+        cudaLaunchAttribute attr[2];
         if (grid) {
             attr[0].id = cudaLaunchAttributeCooperative;
             attr[0].val.cooperative = 1;
@@ -504,8 +505,10 @@ cudaError_t launch_pcg_chip(const DevCase *cases, const PcgGroup &pg, cudaStream
             attr[0].val.clusterDim.y = 1;
             attr[0].val.clusterDim.z = 1;
         }
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization; // as launch_next
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        cfg.numAttrs = grid || prof::g_on ? 1 : 2;
         prof::mark(st, grid ? "k_pcg_grid" : "k_pcg");
         cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
         if (e != cudaSuccess) return e;
