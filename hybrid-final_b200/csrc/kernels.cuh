@@ -40,7 +40,7 @@ struct LaunchCfg {
     int warps_per_block = 4;   // particle kernels: one warp per (species, cell)
     int pcg_block = 512;       // PCG: threads per CTA
     int pcg_cluster_max = 16;  // PCG: upper bound on CTAs per case
-    int move_unroll = 1;       // Move: chunks of 32 loaded per iteration (1: k_move, one-chunk prefetch)
+    int move_unroll = 1;       // Move: ring of 5 (1), 4 (2) or 7 (4) chunks of 32 per warp
     int mcc_cells = 16;        // MCC (Ar): most consecutive cells that share collision batches (1, 2, 4, 8, 16)
 };
 
