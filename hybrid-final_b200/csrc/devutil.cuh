@@ -1,7 +1,7 @@
 // devutil.cuh -- device helpers shared by the step kernels (kernels.cu) and
 // the oxygen-chemistry collision kernel (mcc_oxy.cu): warp bookkeeping, the
 // cross-section lookup and the scattering kinematics of the reference's MCC
-// (src/cuda_mcc.cu:139-201), in the arithmetic the CPU checker repeats.
+// (src/cuda_mcc.cu:139-201), in the arithmetic the CPU oracle repeats.
 #pragma once
 #include <cstdint>
 

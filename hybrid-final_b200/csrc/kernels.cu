@@ -8,7 +8,7 @@
 // phases and cluster-wide (DSMEM) reductions of the dot products.
 //
 // Floating-point contract: this file is compiled with --fmad=false so that
-// every a*b+c is two roundings, exactly as the CPU checker evaluates it; the
+// every a*b+c is two roundings, exactly as the CPU oracle evaluates it; the
 // elementary functions come from hp_math.h, identical on host and device.
 #include <cooperative_groups.h>
 
