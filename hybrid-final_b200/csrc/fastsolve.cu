@@ -22,11 +22,11 @@
 //  * up to FS_CLUSTER_MAX unknowns a cluster runs the whole solve, all passes
 //    and the final residual, with cluster barriers between the phases: the
 //    strips of 16 CTAs keep up with a launch chain of the whole GPU there
-//    (129x65 nodes: a step of 142 us with one launch per
-//    product, 119 us so);
+//    (129x65 nodes: a step of 142 us with one launch per product, 119 us so);
 //    above that each product is a launch of 32 x 32 tiles over the whole GPU, as
-//    a strip's left operand would be read from L2 once per strip there
-//    (that form took 32 us per pair of products at 513x257, two launches 22 us).
+//    a strip's left operand would be read from L2 once per strip there (191x94
+//    nodes: a step of 254 us in a cluster, 232 in tiles; the eight products of a
+//    513x257 solve 127 us in strips over the whole GPU, 119 in tiles).
 #include <cooperative_groups.h>
 
 #include <algorithm>

@@ -1,11 +1,11 @@
 // kernels.cu -- sm_100a kernels of one PIC/MCC step, batched over cases.
 //
-// Work mapping: the particle kernels give one warp to one (case, species,
-// cell); the slots of a cell are contiguous, so each warp access is one or
-// more full 128-byte lines.  The grid kernels give one thread to one node.
-// The Poisson solve runs one thread-block cluster per case and keeps the
-// whole CG iteration inside one launch, with cluster barriers between the
-// phases and cluster-wide (DSMEM) reductions of the dot products.
+// Work mapping: the particle kernels give a (case, species, cell) to one
+// warp, and a warp one or more of them; the slots of a cell are contiguous,
+// so each warp access is one or more full 128-byte lines.  The grid kernels
+// give one thread to one node.  The Poisson solve runs in one launch, on one
+// thread-block cluster per case or on the whole GPU (pcg.cu; k_pcg here for
+// the launch shapes that do not fit on chip).
 //
 // Floating-point contract: this file is compiled with --fmad=false so that
 // every a*b+c is two roundings, exactly as the CPU oracle evaluates it; the
