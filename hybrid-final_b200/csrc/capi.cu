@@ -337,6 +337,7 @@ hp_status build_device(hp_case *c) {
         TRY(dalloc(c, &sp.cnt, C));
         TRY(dalloc(c, &sp.nmov, C));
         TRY(dalloc(c, &sp.dcount, (size_t)C * 9));
+        TRY(dalloc(c, &sp.dslot, (size_t)C * 9));
         TRY(dalloc(c, &h.cw[isp], C));
     }
     TRY(dalloc(c, &h.Ex, G));
@@ -931,7 +932,7 @@ size_t estimate_device_bytes(const hp::Setup &s, const hp_case_opts &o) {
     size_t b = 0;
     for (int k = 0; k < s.nsp; k++) {
         const size_t cap = (size_t)s.cap[k]; // already sized by the cap_per_cell option
-        b += C * cap * 21 + C * (4 + 4 + 36 + 32);         // slots, counts, dcount, corner sums
+        b += C * cap * 21 + C * (4 + 4 + 36 + 36 + 32);    // slots, counts, dcount, dslot, corner sums
     }
     b += nsp * C * (4 + 8 * HP_FAR_BUCKET) + 8 * C * 4;  // far buckets, channel counts
     b += G * (16 * 4 + 8 * 8 + 16 * nsp) + C * 16 + (size_t)s.cond_numr * G * 4;

@@ -11,6 +11,7 @@
 //     cnt[s][c]                         int32   particles resident in cell c
 //     nmov[s][c]                        int32   movers parked at the top of cell c
 //     dcount[s][c*9 + code]             int32   of those, movers to each of the 3x3 cells
+//     dslot[s][c*9 + code]              int32   the slot in that cell at which they start (Sort)
 //   cell c = i*ncy + j for the cell whose lower-left node is (i, j); the
 //   reference indexes the same cell by its node i*ngy + j and strides its
 //   slots by Gsize (src/cuda_Particle.cu:44-52).  Slots of one cell are
@@ -58,6 +59,7 @@ struct DevSpecies {
     int *cnt;
     int *nmov;
     int *dcount; // [C*9] movers per cell and destination code 0..8 (after Move)
+    int *dslot;  // [C*9] first slot of those movers in their destination (after the count pass of Sort)
     int cap;
     float Ascale, q_density, Escale, np2c;
 };

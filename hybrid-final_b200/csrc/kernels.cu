@@ -441,15 +441,17 @@ __global__ void __launch_bounds__(512, MOVE_MINB) k_move(const DevCase *__restri
 // rules were applied by Move, which also counted each cell's movers per
 // destination (dcount).  Two passes, no loop-carried dependency in either:
 //   k_sort_count  (lane per destination cell) runs over the nine counts
-//                addressed to it in source order, puts in the place of each
-//                the slot that source's movers start at, finishes the far
-//                movers and writes the new count;
+//                addressed to it in source order, writes for each the slot
+//                that source's movers start at, finishes the far movers and
+//                writes the new count;
 //   k_sort_push  (warp per source cells) puts each near mover at its start
 //                slot + its rank among the source's movers to that cell.
-// A (source, code) count is addressed to one cell, so the plan replaces it in
-// place, and a source finds the nine slots it needs side by side.  (Summing
+// A (source, code) count is addressed to one cell, so its start slot has one
+// writer, and a source finds the nine slots it needs side by side.  (Summing
 // the counts of the lower-index sources in the push instead takes 81 loads and
-// index computations per source cell.)
+// index computations per source cell.)  The slots have an array of their own:
+// Move's counts stay what they are, so that a second sort with no Move in
+// between plans from counts again, not from slots.
 constexpr int SORT_MAXW = 16; // warps per block, at most
 
 constexpr int SORT_MINB = 2; // resident 512-thread blocks per SM the register budget is set for
@@ -544,7 +546,7 @@ __global__ void __launch_bounds__(SORT_MAXW * 32, SORT_MINB) k_sort_push(const D
             const int Di = i + lane / 3 - 1, Dj = j + lane % 3 - 1;
             if (Di >= 0 && Di < d.ncx && Dj >= 0 && Dj < ncy) {
                 D = Di * ncy + Dj;
-                at = sp.dcount[(size_t)c * 9 + lane];
+                at = sp.dslot[(size_t)c * 9 + lane];
                 lim = sp.cap - sp.nmov[D];
             }
         }
@@ -635,7 +637,7 @@ __global__ void __launch_bounds__(SORT_MAXW * 32) k_sort_count(const DevCase *__
 #pragma unroll
         for (int q = 0; q < 9; q++)
             if (in[q]) {
-                sp.dcount[(size_t)(c + (q / 3 - 1) * ncy + (q % 3 - 1)) * 9 + (8 - q)] = out;
+                sp.dslot[(size_t)(c + (q / 3 - 1) * ncy + (q % 3 - 1)) * 9 + (8 - q)] = out;
                 out += in[q];
             }
     }

@@ -77,6 +77,55 @@ def test_operators_bit_exact(move_mode, cells):
     case.close()
 
 
+def test_sorts_in_a_row():
+    """SortBoundary once more with no Move in between files the parked movers again, source cells in increasing
+    order, and stays inside the cells however often it is called."""
+    ncx, ncy, cs = 9, 7, 3.125e-4
+    deck = ccp_deck(ncx + 1, ncy + 1, ncx * cs, ncy * cs, ppc=4)
+    case = hpic.Case(deck, seed=3, field_mode=1, move_mode=1, cap_per_cell=1024)
+    rng = np.random.default_rng(5)
+    C = ncx * ncy
+    counts = np.array([COUNTS[k % 6] for k in range(C)], np.int32)
+    n = int(counts.sum())
+    x, y, *v = (rng.random(n, dtype=np.float32) for _ in range(5))
+    v = [(a * 2 - 1) * np.float32(0.9 * cs / float(case.info.dt)) for a in v]  # under one cell per step: near movers only
+    for s in range(2):
+        case.set_particles(s, counts, x, y, *v)
+    case.Move()
+    moved = [case.movers(s) for s in range(2)]
+    assert all(m[0].sum() > 0 for m in moved)
+    case.SortBoundary()
+    want = [case.particles(s) for s in range(2)]
+    for _ in range(12):
+        case.SortBoundary()
+        for s in range(2):
+            mc, ma, code = moved[s]
+            at = np.concatenate([[0], np.cumsum(mc)])
+            pc, pa = want[s]
+            start = np.concatenate([[0], np.cumsum(pc)])
+            new_c, new_a = np.zeros_like(pc), [[] for _ in range(5)]
+            for c in range(C):
+                i, j = divmod(c, ncy)
+                own = np.arange(start[c], start[c + 1])
+                add = []
+                for si in range(max(i - 1, 0), min(i + 2, ncx)):
+                    for sj in range(max(j - 1, 0), min(j + 2, ncy)):
+                        src = si * ncy + sj
+                        q = np.arange(at[src], at[src + 1])
+                        add.append(q[code[q] == (i - si + 1) * 3 + (j - sj + 1)])
+                add = np.concatenate(add)
+                new_c[c] = own.size + add.size
+                for a in range(5):
+                    new_a[a] += [pa[a][own], ma[a][add]]
+            want[s] = new_c, [np.concatenate(a) for a in new_a]
+            got_c, got_a = case.particles(s)
+            assert np.array_equal(got_c, want[s][0])
+            for a in range(5):
+                assert np.array_equal(bits(got_a[a]), bits(want[s][1][a]))
+    assert case.status() == 0
+    case.close()
+
+
 def test_mcc_groups_of_cells():
     """Collision groups of 5 cells (16,200 cells, the last group cut short), against the oracle, and a group that
     holds the end of one case and the start of the next in a batch."""
