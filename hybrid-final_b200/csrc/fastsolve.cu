@@ -384,11 +384,6 @@ __global__ void __launch_bounds__(32) k_fs_norm(const DevCase *__restrict__ case
 
 inline unsigned nblocks(long long threads, int per) { return (unsigned)((threads + per - 1) / per); }
 
-cudaError_t allow_smem(const void *fn, size_t bytes) {
-    return bytes > 48 * 1024 ? cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)
-                             : cudaSuccess;
-}
-
 } // namespace
 
 size_t fs_cluster_smem(int nx, int ny) {

@@ -2006,12 +2006,18 @@ cudaError_t launch_move(const DevCase *cases, const int *item_start, int ncases,
     if (items <= 0) return cudaSuccess;
     const int tpb = 32 * std::min(std::max(lc.warps_per_block, 1), 16);
     const unsigned nb = blocks_for((long long)items * 32, tpb);
-    prof::mark(st, "k_move");
-    const size_t slot = (size_t)(tpb / 32) * MOVE_SLOT * sizeof(float);
-    if (lc.move_unroll == 2) launch_next(k_move<MOVE_RING - 1>, nb, tpb, (MOVE_RING - 1) * slot, st, cases, item_start, ncases, items);
-    else if (lc.move_unroll == 4) launch_next(k_move<MOVE_RING + 2>, nb, tpb, (MOVE_RING + 2) * slot, st, cases, item_start, ncases, items);
-    else launch_next(k_move<MOVE_RING>, nb, tpb, MOVE_RING * slot, st, cases, item_start, ncases, items);
-    return cudaGetLastError();
+    // a slot is 640 bytes: 16 warps with 5 slots take 50 KB, with 7 slots 70 KB
+    auto move = [&](auto kernel, int slots) {
+        const size_t smem = (size_t)(tpb / 32) * slots * MOVE_SLOT * sizeof(float);
+        const cudaError_t e = allow_smem((const void *)kernel, smem);
+        if (e != cudaSuccess) return e;
+        prof::mark(st, "k_move");
+        launch_next(kernel, nb, tpb, smem, st, cases, item_start, ncases, items);
+        return cudaGetLastError();
+    };
+    if (lc.move_unroll == 2) return move(k_move<MOVE_RING - 1>, MOVE_RING - 1);
+    if (lc.move_unroll == 4) return move(k_move<MOVE_RING + 2>, MOVE_RING + 2);
+    return move(k_move<MOVE_RING>, MOVE_RING);
 }
 
 cudaError_t launch_power(DevCase *cases, int ncases, cudaStream_t st) {

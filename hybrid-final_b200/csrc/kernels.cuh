@@ -36,6 +36,13 @@ inline cudaError_t launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// Dynamic shared memory past the 48 KB that a launch may ask for unannounced;
+// per device, so before every such launch.
+inline cudaError_t allow_smem(const void *fn, size_t bytes) {
+    return bytes > 48 * 1024 ? cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)
+                             : cudaSuccess;
+}
+
 struct LaunchCfg {
     int warps_per_block = 4;   // particle kernels: one warp per (species, cell)
     int pcg_block = 512;       // PCG: threads per CTA
