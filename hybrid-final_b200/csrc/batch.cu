@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "capi_internal.hpp"
+#include "side_work.hpp"
 
 using namespace hp;
 using hpi::cuda_fail;
@@ -155,15 +156,26 @@ void batch_dev_free(BatchDev &b) {
 
 hp_status run_step(const BatchDev &b, const LaunchCfg &lc, int gas, cudaStream_t st) {
     CK(launch_advance(b.d_cases, b.n, st));
-    if (b.fluid.any) CK(fluid_begin(b.d_cases, b.n, b.fluid, b.fluid_fork, st));
-    const std::vector<PcgGroup> g = b.groups(lc.pcg_cluster_max, lc.pcg_block);
-    CK(launch_field(b.d_cases, b.d_node, b.n, b.n_node, g.data(), (int)g.size(), &b.fast.plan, st, b.circuit));
-    CK(launch_move(b.d_cases, b.d_part, b.n, b.n_part, lc, st));
-    CK(launch_sort(b.d_cases, b.d_part, b.n, b.n_part, lc, st, b.surface));
-    if (gas != GAS_AR) CK(launch_mcc_oxy(b.d_cases, b.d_cell, b.n, b.n_cell, gas, st));
-    else CK(launch_mcc_ar(b.d_cases, b.d_cell, b.n, b.n_cell, lc, st));
-    CK(launch_deposit(b.d_cases, b.d_part, b.d_node, b.n, b.n_part, b.n_node, lc, st, b.max_smt));
-    if (b.fluid.any) CK(fluid_end(b.d_cases, b.d_node, b.n, b.n_node, b.fluid, b.fluid_fork, st));
+    auto begin = [&]() -> hp_status {
+        if (b.fluid.any) CK(fluid_begin(b.d_cases, b.n, b.fluid, b.fluid_fork, st));
+        return HP_OK;
+    };
+    auto body = [&]() -> hp_status {
+        const std::vector<PcgGroup> g = b.groups(lc.pcg_cluster_max, lc.pcg_block);
+        CK(launch_field(b.d_cases, b.d_node, b.n, b.n_node, g.data(), (int)g.size(), &b.fast.plan, st, b.circuit));
+        CK(launch_move(b.d_cases, b.d_part, b.n, b.n_part, lc, st));
+        CK(launch_sort(b.d_cases, b.d_part, b.n, b.n_part, lc, st, b.surface));
+        if (gas != GAS_AR) CK(launch_mcc_oxy(b.d_cases, b.d_cell, b.n, b.n_cell, gas, st));
+        else CK(launch_mcc_ar(b.d_cases, b.d_cell, b.n, b.n_cell, lc, st));
+        CK(launch_deposit(b.d_cases, b.d_part, b.d_node, b.n, b.n_part, b.n_node, lc, st, b.max_smt));
+        return HP_OK;
+    };
+    auto end = [&]() -> hp_status {
+        if (b.fluid.any) CK(fluid_end(b.d_cases, b.d_node, b.n, b.n_node, b.fluid, b.fluid_fork, st));
+        return HP_OK;
+    };
+    const hp_status s = with_side_work(HP_OK, begin, body, end, [&] { fluid_join(b.fluid, b.fluid_fork, st); });
+    if (s != HP_OK) return s;
     CK(launch_accumulate(b.d_cases, b.d_node, b.n, b.n_node, st));
     if (b.any_eedf) CK(launch_eedf(b.d_cases, b.d_cell, b.n, b.n_cell, st));
     if (b.power) CK(launch_power(b.d_cases, b.n, st));
@@ -179,11 +191,15 @@ hp_status capture(hp_batch *b) {
         cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;
     }
-    cudaGraph_t g;
+    cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(b->own, cudaStreamCaptureModeThreadLocal));
     hp_status s1 = hpi::run_step(b->dev, b->lc, b->gas, b->own);
     cudaError_t e = cudaStreamEndCapture(b->own, &g);
-    if (s1 != HP_OK) return s1;
+    if (s1 != HP_OK) {
+        if (g) cudaGraphDestroy(g);
+        cudaGetLastError(); // the capture's own error, after the step's
+        return s1;
+    }
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
     b->graph_kernels = hpi::count_kernel_nodes(g);
     e = cudaGraphInstantiate(&b->graph, g, 0);
@@ -297,7 +313,8 @@ hp_status hp_batch_get_tune(hp_batch *b, hp_tune *t) {
 
 // Times candidate launch shapes on the batch itself.  Every case's device
 // state is copied aside first and restored after each trial, so the batch
-// resumes exactly where it stood.
+// resumes exactly where it stood.  A trial that fails has joined its fluid
+// sweeps (run_step), so the restore is ordered behind them too.
 hp_status hp_batch_autotune(hp_batch *b, void *stream) {
     if (!b) return HP_ERR_ARG;
     CK(cudaSetDevice(b->device));

@@ -10,6 +10,7 @@
 
 #include "capi_internal.hpp"
 #include "prof.cuh"
+#include "side_work.hpp"
 
 using namespace hp;
 
@@ -44,6 +45,7 @@ int count_kernel_nodes(cudaGraph_t g) {
 
 hp_status cuda_fail(cudaError_t e, const char *what) {
     set_error(std::string(what) + ": " + cudaGetErrorString(e));
+    cudaGetLastError(); // reported here: not by the next launch's check as well
     return HP_ERR_CUDA;
 }
 
@@ -615,19 +617,23 @@ hp_status op_deposit(hp_case *c, cudaStream_t st, bool smooth) {
 hp_status one_step(hp_case *c, cudaStream_t st) {
     cudaError_t e = launch_advance(c->d_case, 1, st);
     if (e != cudaSuccess) return cuda_fail(e, "advance");
-    if (c->fplan_fluid.any) {
-        e = fluid_begin(c->d_case, 1, c->fplan_fluid, c->fl_fork, st);
-        if (e != cudaSuccess) return cuda_fail(e, "fluid");
-    }
-    TRY(op_field(c, st));
-    TRY(op_move(c, st));
-    TRY(op_sort(c, st));
-    TRY(op_mcc(c, st));
-    TRY(op_deposit(c, st, true));
-    if (c->fplan_fluid.any) {
-        e = fluid_end(c->d_case, c->d_items + 4, 1, c->s.Gsize, c->fplan_fluid, c->fl_fork, st);
-        if (e != cudaSuccess) return cuda_fail(e, "fluid");
-    }
+    auto fluid = [&](cudaError_t f) { return f == cudaSuccess ? HP_OK : cuda_fail(f, "fluid"); };
+    auto begin = [&]() -> hp_status {
+        return c->fplan_fluid.any ? fluid(fluid_begin(c->d_case, 1, c->fplan_fluid, c->fl_fork, st)) : HP_OK;
+    };
+    auto body = [&]() -> hp_status {
+        TRY(op_field(c, st));
+        TRY(op_move(c, st));
+        TRY(op_sort(c, st));
+        TRY(op_mcc(c, st));
+        return op_deposit(c, st, true);
+    };
+    auto end = [&]() -> hp_status {
+        return c->fplan_fluid.any
+                   ? fluid(fluid_end(c->d_case, c->d_items + 4, 1, c->s.Gsize, c->fplan_fluid, c->fl_fork, st))
+                   : HP_OK;
+    };
+    TRY(with_side_work(HP_OK, begin, body, end, [&] { fluid_join(c->fplan_fluid, c->fl_fork, st); }));
     e = launch_accumulate(c->d_case, c->d_items + 4, 1, c->s.Gsize, st);
     if (e == cudaSuccess && c->h.eedf_every > 0) e = launch_eedf(c->d_case, c->d_items + 2, 1, c->s.Csize, st);
     if (e == cudaSuccess && c->h.pw) e = launch_power(c->d_case, 1, st);
@@ -1017,11 +1023,15 @@ hp_status hp_step(hp_case *c, int nsteps, void *stream) {
         CK(cudaEventRecord(ev, st));
         CK(cudaStreamWaitEvent(c->own_stream, ev, 0));
         CK(cudaEventDestroy(ev));
-        cudaGraph_t g;
+        cudaGraph_t g = nullptr;
         CK(cudaStreamBeginCapture(c->own_stream, cudaStreamCaptureModeThreadLocal));
         hp_status s1 = one_step(c, c->own_stream);
         cudaError_t e = cudaStreamEndCapture(c->own_stream, &g);
-        if (s1 != HP_OK) return s1;
+        if (s1 != HP_OK) {
+            if (g) cudaGraphDestroy(g);
+            cudaGetLastError(); // the capture's own error, after the step's
+            return s1;
+        }
         if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
         c->graph_kernels = hpi::count_kernel_nodes(g);
         e = cudaGraphInstantiate(&c->graph, g, 0);

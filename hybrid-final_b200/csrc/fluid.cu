@@ -380,4 +380,12 @@ cudaError_t fluid_end(const DevCase *cases, const int *node_items, int ncases, i
     return launch_fluid_diag(cases, node_items, ncases, n_node_items, fp, st);
 }
 
+// the event is recorded here as well: a begin that failed has not done so
+cudaError_t fluid_join(const FluidPlan &fp, const FluidFork &f, cudaStream_t st) {
+    if (!forked(fp, f)) return cudaSuccess;
+    cudaError_t e = cudaEventRecord(f.join, f.side);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(st, f.join, 0);
+    return e;
+}
+
 } // namespace hp

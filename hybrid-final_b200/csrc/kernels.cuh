@@ -156,6 +156,7 @@ cudaError_t launch_fluid(const DevCase *cases, const int *node_items, int ncases
 // and fluid_end (before the accumulation) joins it back and runs the
 // averaging cycle.  Without a side stream, or while a per-kernel profile is
 // recorded, fluid_begin does nothing and fluid_end runs launch_fluid.
+// fluid_join, for a step that fails in between, only joins (side_work.hpp).
 struct FluidFork {
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
@@ -165,5 +166,6 @@ void fluid_fork_destroy(FluidFork &f);
 cudaError_t fluid_begin(const DevCase *cases, int ncases, const FluidPlan &fp, const FluidFork &f, cudaStream_t st);
 cudaError_t fluid_end(const DevCase *cases, const int *node_items, int ncases, int n_node_items, const FluidPlan &fp,
                       const FluidFork &f, cudaStream_t st);
+cudaError_t fluid_join(const FluidPlan &fp, const FluidFork &f, cudaStream_t st);
 
 } // namespace hp
