@@ -89,8 +89,10 @@ struct PcgGroup {
     int max_per, max_ngy; // most nodes per CTA and grid rows of its cases
 };
 // the solve with its state on chip (pcg.cu); done = false where the group's
-// launch shape is outside its range
-cudaError_t launch_pcg_chip(const DevCase *cases, const PcgGroup &pg, cudaStream_t st, bool &done);
+// launch shape is outside its range.  polls: reads of one word before a wait of
+// the whole-GPU form gives up (each is an L2 round trip: seconds)
+cudaError_t launch_pcg_chip(const DevCase *cases, const PcgGroup &pg, cudaStream_t st, bool &done,
+                            int polls = 1 << 22);
 // field_mode 2 (fastsolve.cu): refinement passes with the separable inverse
 constexpr int FS_CHUNK = 1024;  // nodes per CTA of the final residual pass; a case's fs_res holds
                                 // 2 + 2 * ceil(G / FS_CHUNK) doubles

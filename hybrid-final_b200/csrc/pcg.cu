@@ -47,8 +47,14 @@ using namespace dv;
 constexpr int MAXW = 16;      // warps per CTA
 constexpr int MAXC = 16;      // CTAs of a cluster
 constexpr int GRID_MAX = 512; // CTAs of the whole-GPU form
-// polls of one word before a wait gives up (each is an L2 round trip: seconds)
-constexpr int POLL_LIMIT = 1 << 22;
+// A solve numbers its exchanges from past every number that the one before can
+// have used.  After a wait that gave up the CTAs need not have stopped at the
+// same number: one can have finished the exchange that another gave up on, and
+// from its own last finished exchange a CTA sends at most three more before it
+// leaves (in mode 1, the sum that gives up and the two of the next residual)
+// and publishes its edges under at most the next number.  The stored number is
+// CTA 0's last; words up to three past it may lie in the inboxes.
+constexpr unsigned EXCHANGE_GAP = 8;
 
 __device__ __forceinline__ unsigned long long ld_word(const unsigned long long *p) {
     unsigned long long v;
@@ -62,8 +68,8 @@ __device__ __forceinline__ unsigned long long tagged(unsigned tag, unsigned data
     return ((unsigned long long)tag << 32) | data;
 }
 // the data of a word once it carries `tag`; false when it never did
-__device__ __forceinline__ bool poll_word(const unsigned long long *p, unsigned tag, unsigned &data) {
-    for (int k = 0; k < POLL_LIMIT; k++) {
+__device__ __forceinline__ bool poll_word(const unsigned long long *p, unsigned tag, int polls, unsigned &data) {
+    for (int k = 0; k < polls; k++) {
         const unsigned long long v = ld_word(p);
         if ((unsigned)(v >> 32) == tag) {
             data = (unsigned)v;
@@ -79,8 +85,8 @@ __device__ __forceinline__ void st_double(unsigned long long *p, unsigned tag, d
                  "l"(tagged(tag, (unsigned)(u >> 32)))
                  : "memory");
 }
-__device__ __forceinline__ bool poll_double(const unsigned long long *p, unsigned tag, double &v) {
-    for (int k = 0; k < POLL_LIMIT; k++) {
+__device__ __forceinline__ bool poll_double(const unsigned long long *p, unsigned tag, int polls, double &v) {
+    for (int k = 0; k < polls; k++) {
         unsigned long long a, b;
         asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
         if ((unsigned)(a >> 32) == tag && (unsigned)(b >> 32) == tag) {
@@ -109,7 +115,7 @@ template <> struct Shared<true> { // the whole GPU's
 // which the neighbours read.
 template <bool GRID, int K>
 __global__ void __launch_bounds__(512, 1) k_pcg_chip(const DevCase *__restrict__ cases, const int *__restrict__ list,
-                                                  int nlist, int max_per, int max_ngy) {
+                                                  int nlist, int max_per, int max_ngy, int polls) {
     enter_kernel();
     extern __shared__ float dyn[];
     __shared__ Shared<GRID> sh;
@@ -131,7 +137,7 @@ __global__ void __launch_bounds__(512, 1) k_pcg_chip(const DevCase *__restrict__
 
     // ---- exchanges
     int parity = 0;
-    unsigned tag = GRID ? *d.pcg_seq : 0u; // the last exchange of the previous solve
+    unsigned tag = GRID ? *d.pcg_seq + EXCHANGE_GAP : 0u; // pcg_seq: the last exchange of the solve before
     bool gave_up = false;
     if constexpr (GRID)
         if (t == 0) sh.gave_up = 0;
@@ -165,7 +171,7 @@ __global__ void __launch_bounds__(512, 1) k_pcg_chip(const DevCase *__restrict__
         if constexpr (GRID) {
             const unsigned long long *in = d.pcg_slot + (size_t)(tag & 1u) * 2 * CS * CS + 2 * (size_t)rank * CS;
             for (int q = t; q < CS; q += T)
-                if (!poll_double(in + 2 * q, tag, sh.cta[q])) sh.gave_up = 1;
+                if (!poll_double(in + 2 * q, tag, polls, sh.cta[q])) sh.gave_up = 1;
             if (fence) __threadfence();
             __syncthreads();
             if (t == 0) { // 16 loads ahead of the chain of additions
@@ -264,7 +270,7 @@ __global__ void __launch_bounds__(512, 1) k_pcg_chip(const DevCase *__restrict__
     auto halo_r = [&](int q) -> float {
         if constexpr (GRID) {
             unsigned u = 0;
-            if (!poll_word(hw[q], tag, u)) sh.gave_up = 1;
+            if (!poll_word(hw[q], tag, polls, u)) sh.gave_up = 1;
             return __uint_as_float(u);
         } else {
             const int e = t + q * T;
@@ -464,7 +470,7 @@ const Variant VARIANTS[] = {
 // (128 registers at 512 threads) and whose halo is at most two nodes per
 // thread; a launch shape with fewer, wider CTAs than that (hp_tune) keeps
 // k_pcg.  Shared memory stays below 48 KB: 4 x (2 x 4096 + 2 x 512) bytes.
-cudaError_t launch_pcg_chip(const DevCase *cases, const PcgGroup &pg, cudaStream_t st, bool &done) {
+cudaError_t launch_pcg_chip(const DevCase *cases, const PcgGroup &pg, cudaStream_t st, bool &done, int polls) {
     done = false;
     const bool grid = pg.cluster > 16;
     // several CTAs own more than 1000 nodes each, so a halo reaches no further than the CTAs next to its own
@@ -489,7 +495,7 @@ cudaError_t launch_pcg_chip(const DevCase *cases, const PcgGroup &pg, cudaStream
     for (int k = 0; k < (grid ? pg.n : 1); k++) { // the whole-GPU form: one case per launch
         const int *list = pg.list + k;
         int nlist = grid ? 1 : pg.n, per = pg.max_per, ngy = pg.max_ngy;
-        void *args[] = {(void *)&cases, (void *)&list, (void *)&nlist, (void *)&per, (void *)&ngy};
+        void *args[] = {(void *)&cases, (void *)&list, (void *)&nlist, (void *)&per, (void *)&ngy, (void *)&polls};
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)(grid ? pg.cluster : pg.n * pg.cluster), 1, 1);
         cfg.blockDim = dim3((unsigned)pg.block, 1, 1);

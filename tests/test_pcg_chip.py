@@ -3,6 +3,8 @@ CTA to a 16-CTA cluster to the whole GPU, halos of one and two nodes per thread,
 it that keep k_pcg.  Every solve has to give the oracle's bits (the oracle repeats the reduction tree of the same
 number of CTAs and threads)."""
 import ctypes as C
+import os
+import subprocess
 
 import numpy as np
 import pytest
@@ -55,3 +57,21 @@ def test_solve_bit_exact(nx, ny, block, cluster, mode):
         assert case.pcg_iters()[0] == o.counters()[2][0]
     assert case.status() == 0
     case.close()
+
+
+def test_solve_after_one_whose_waits_gave_up(tmp_path):
+    """The whole-GPU solve with no polls allowed returns with HP_STATUS_WAIT_TIMEOUT, and the solve after it takes none
+    of the words that such a solve can leave behind (tests/pcg_words.cu)."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    src = os.path.join(here, "..", "hybrid-final_b200", "csrc")
+    exe = str(tmp_path / "pcg_words")
+    subprocess.run(["nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-O2", "-std=c++17", "--fmad=false", "-I", src,
+                    "-I", os.path.join(here, "..", "include"), os.path.join(here, "pcg_words.cu"),
+                    os.path.join(src, "prof.cu"), "-o", exe], check=True)
+    lines = subprocess.run([exe], capture_output=True, text=True, timeout=120).stdout.splitlines()
+    assert len(lines) == 2, lines
+    for line in lines:
+        f = line.split()
+        assert f[2:9] == ["ran", "1", "gave_up", "1", "same", "1", "iterations"], line
+        assert f[9] == f[10] and int(f[9]) > 5, line
+        assert f[11:] == ["nonzero", "1", "status", "0", "0"], line

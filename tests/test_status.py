@@ -4,9 +4,9 @@ The reference has no error reporting: a CUDA error calls exit()
 (src/cuda_main.cu:2-9) and an overfull cell is halved in place by ReArgPtcls
 (src/cuda_Sortboundary.cu:23-40).  Here the kernels set a bit of the case's
 status word and carry on with defined results; each test drives one
-condition with ordinary inputs and checks the bit.  HP_STATUS_WAIT_TIMEOUT is
-never raised: no kernel of this library spins on a flag (the cluster
-barriers are cluster.sync())."""
+condition with ordinary inputs and checks the bit.  HP_STATUS_WAIT_TIMEOUT,
+which the whole-GPU PCG sets when a bounded poll gives up, has its test in
+test_pcg_chip.py (a solve that may not poll)."""
 import numpy as np
 import pytest
 
