@@ -25,12 +25,15 @@ __device__ __forceinline__ int find_case(const int *start, int n, int w) {
     return lo;
 }
 
-// First statement of every kernel of a step: wait until the kernel before it
-// in the stream has finished and its writes are visible (nothing is read
-// before), then let the next one be put on the SMs that have room, where it
-// waits in the same place.  With a launch by launch_next (kernels.cuh) the
-// next kernel's launch latency then passes while this one runs; without it
-// both instructions do nothing.
+// First statement of every kernel that is launched by launch_next (kernels.cuh)
+// or with its attribute: wait until the kernel before it in the stream has
+// finished and its writes are visible (nothing is read before), then let the
+// next one be put on the SMs that have room, if it was launched so too, where
+// it waits in the same place; its launch latency then passes while this one
+// runs.  Whether the wait has anything to wait for is up to this kernel's own
+// launch, whether anything starts early is up to the next one's: in plain
+// stream order a kernel starts after all that is before it, and one launched
+// plainly still lets a successor with the attribute start early.
 __device__ __forceinline__ void enter_kernel() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -286,7 +286,8 @@ __global__ void __launch_bounds__(256) k_fs_resid(const DevCase *__restrict__ ca
 // in flight (with one slice read ahead into registers a k step took 57
 // cycles at 513x257, the shared-memory reads and the arithmetic each ask for
 // 16).  Lanes run along the edge that the result is stored along.
-constexpr int GT = 32, GK = 32, GEMM_STAGES = 6, GEMM_THREADS = 256;
+constexpr int GT = FS_TILE, GK = 32, GEMM_STAGES = 6, GEMM_THREADS = 256; // the host counts FS_TILE tiles
+static_assert(GT == 32, "16 x 16 threads of 2 x 2 outputs, copies of 8 x 16 bytes per row");
 
 template <int S>
 __global__ void __launch_bounds__(GEMM_THREADS) k_gemm(const DevCase *__restrict__ cases,

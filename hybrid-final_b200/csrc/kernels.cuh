@@ -10,10 +10,13 @@
 
 namespace hp {
 
-// A kernel that begins with enter_kernel(), launched so that its start
-// overlaps the end of the kernel before it in the stream (programmatic
-// dependent launch; captured into a graph as such an edge).  Not while a
-// per-kernel profile is recorded: its marks bracket whole kernels.
+// A kernel launched so that its start overlaps the end of the kernel before it
+// in the stream (programmatic dependent launch; captured into a graph as such
+// an edge).  Only for kernels that begin with enter_kernel(): without its wait
+// a kernel would run beside the one whose results it reads.  k_fs_resid,
+// k_gemm, k_pcg, k_fluid_sweep and k_fluid_diag have none and stay in plain
+// stream order, as do the loader's and the allocation-free deposit's kernels.
+// Not while a per-kernel profile is recorded: its marks bracket whole kernels.
 // Only for launches of up to about half of the threads that fit on the chip: a
 // launch's start is then a part of its time.  Measured on a B200, a step in
 // plain stream order, with this rule, and with every launch so: 66.0, 63.7
@@ -44,7 +47,7 @@ inline cudaError_t allow_smem(const void *fn, size_t bytes) {
 }
 
 struct LaunchCfg {
-    int warps_per_block = 4;   // particle kernels: one warp per (species, cell)
+    int warps_per_block = 4;   // warps per CTA of Move, Deposit's cells and (at least 8) the re-binning
     int pcg_block = 512;       // PCG: threads per CTA
     int pcg_cluster_max = 16;  // PCG: upper bound on CTAs per case
     int move_unroll = 1;       // Move: ring of 5 (1), 4 (2) or 7 (4) chunks of 32 per warp
@@ -66,7 +69,7 @@ cudaError_t launch_power(DevCase *cases, int ncases, cudaStream_t st);
 cudaError_t launch_sort(const DevCase *cases, const int *item_start, int ncases, int items, const LaunchCfg &lc,
                         cudaStream_t st, bool surface);
 // MCC, Ar set (src/cuda_mcc.cu:97-106, src/cuda_mccAr.cu:41-232)
-// MCC of the Ar/O2 (gas 2) reaction set, one warp per cell (mcc_oxy.cu)
+// MCC of the Ar/O2 (gas 2) reaction set, one warp per up to four cells (mcc_oxy.cu)
 cudaError_t launch_mcc_oxy(const DevCase *cases, const int *item_start, int ncases, int items, int gas,
                            cudaStream_t st);
 cudaError_t launch_mcc_ar(const DevCase *cases, const int *item_start, int ncases, int items, const LaunchCfg &lc,

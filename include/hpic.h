@@ -397,7 +397,9 @@ hp_status hp_batch_step(hp_batch *b, int nsteps, void *stream);
 hp_status hp_batch_step_kernels(const hp_batch *b, int *n);
 /* Per-phase launch shape chosen by the autotuner (hp_batch_autotune) or set here. */
 typedef struct hp_tune {
-    int warps_per_block_particles; /* Move/Sort/Deposit: warps per CTA (one warp per cell), 1..16 */
+    int warps_per_block_particles; /* Move, Deposit and (at least 8) Sort: warps per CTA, 1..16.  A warp takes one
+                                      (species, cell) in Move, four in Deposit, one to four in Sort's push and 32
+                                      in its count */
     int pcg_block;                 /* PCG: threads per CTA */
     int pcg_cluster_max;           /* PCG: largest cluster per case */
     int move_unroll;               /* Move: ring of 32-particle chunks per warp: 1 (5 slots), 2 (4) or 4 (7) */
