@@ -19,7 +19,9 @@ def bits(a):
 
 
 @pytest.mark.parametrize("move_mode", [0, 1])
-@pytest.mark.parametrize("cells", [(8, 6), (13, 7)])  # 96 and 182 (species, cell) items: whole and cut groups
+# 96 and 182 (species, cell) items: whole and cut groups of four in the deposit, one item per warp in the sort's push;
+# 10,706 and 19,866 items: groups of three and of four there too, the last one cut (4,736 warps are resident)
+@pytest.mark.parametrize("cells", [(8, 6), (13, 7), (101, 53), (129, 77)])
 def test_operators_bit_exact(move_mode, cells):
     ncx, ncy = cells
     cs = 3.125e-4
