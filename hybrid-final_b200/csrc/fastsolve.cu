@@ -25,8 +25,14 @@
 //    (129x65 nodes: a step of 142 us with one launch per product, 119 us so);
 //    above that each product is a launch of 32 x 32 tiles over the whole GPU, as
 //    a strip's left operand would be read from L2 once per strip there (191x94
-//    nodes: a step of 254 us in a cluster, 232 in tiles; the eight products of a
-//    513x257 solve 127 us in strips over the whole GPU, 119 in tiles).
+//    nodes, which the present cluster form does not take: a step of 254 us in
+//    an earlier one, 232 in tiles; the eight products of a 513x257 solve 127 us in
+//    strips over the whole GPU, 119 in tiles).  The line lies short of where the
+//    two would meet: a step with 10 particles per cell takes, cluster and
+//    tiles, 90 and 103 us at 8,127 unknowns, 95 and 108 at 9,730, and, past the
+//    line, 99 and 110 at 10,400, 105 and 115 at 11,325, 117 and 121 at 12,000
+//    (240x52 nodes), 116 and 121 at 13,203, 129 and 135 at 16,320, about the most
+//    that the cluster form's other limits admit (fs_cluster_ctas).
 #include <cooperative_groups.h>
 
 #include <algorithm>

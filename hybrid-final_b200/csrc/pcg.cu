@@ -452,6 +452,14 @@ __global__ void __launch_bounds__(512, 1) k_pcg_chip(const DevCase *__restrict__
     if (!GRID) cl.sync();
 }
 
+// The forms: 1, 2 and 4 nodes per thread; 5, which is what a grid of 2^a + 1
+// by 2^b + 1 nodes comes to (65x33, 129x65 and 257x129 nodes: 1, 4 and 16 CTAs
+// of 2,073 to 2,145 nodes at 512 threads, where 4 would miss by a few); and 8,
+// the most that 128 registers hold at 512 threads (it spills 56 bytes, 88 on the
+// whole GPU, the others up to 8).  A CTA of 6 or 7 nodes per thread runs the form
+// for 8.  Forms of their own would take, us per iteration at 6 and 7 nodes: one
+// CTA 4.1 and 5.9 against 6.2 and 6.7, a cluster of 16 5.7 and 7.5 against 7.9
+// and 8.3 (k_pcg takes about 12), for 1.9 MB of code; they are not built.
 struct Variant {
     int k;
     const void *cluster, *grid;
@@ -469,7 +477,11 @@ const Variant VARIANTS[] = {
 // The on-chip form takes a group whose CTAs own at most 8 nodes per thread
 // (128 registers at 512 threads) and whose halo is at most two nodes per
 // thread; a launch shape with fewer, wider CTAs than that (hp_tune) keeps
-// k_pcg.  Shared memory stays below 48 KB: 4 x (2 x 4096 + 2 x 512) bytes.
+// k_pcg.  The halo rule holds for a group as a whole: a grid of more rows than
+// threads per CTA (513x257 nodes with hp_tune.pcg_block 128 or 256) takes
+// k_pcg, and with it its whole group (263x251 nodes: 18 us per iteration at 192
+// threads, 24 at 128).
+// Shared memory stays below 48 KB: 4 x (2 x 4096 + 2 x 512) bytes.
 cudaError_t launch_pcg_chip(const DevCase *cases, const PcgGroup &pg, cudaStream_t st, bool &done, int polls) {
     done = false;
     const bool grid = pg.cluster > 16;
